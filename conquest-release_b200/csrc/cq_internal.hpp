@@ -10,6 +10,7 @@
 #include <functional>
 #include <map>
 #include <memory>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -206,7 +207,7 @@ struct ProductPlan {
   DevBuf<int2> pairs;             // [n_pairs] (x block, b block)
   int n_tiles = 0;                // row tiles of the staged 4x4 kernel: (q0, q1, x row first, x row end)
   DevBuf<int4> tiles;
-  DevBuf<int> order;              // output blocks by descending pair count (warp-staged 4x4 kernel)
+  DevBuf<int> order;              // output blocks by descending pair count (staged kernels)
   int tuned = -1;                 // FP64 kernel variant chosen by the autotuner (-1: not tuned yet)
   float tune_ms[7] = {0, 0, 0, 0, 0, 0, 0};
 };
@@ -318,13 +319,14 @@ struct System {
                                   // 2 = one thread per block with the operand row staged in shared memory,
                                   // 3 = one thread per block with warp-cooperative staging of the operand blocks,
                                   // 5 = four lanes per block, 6 = one thread per block with bulk-copy staging;
-                                  // other block sizes: 0 = generic warp per block, 4 = warp per block with
-                                  // 4 x 2 register tiles per lane
+                                  // other block sizes: 0 = generic warp per block, 4 = two or four blocks per
+                                  // warp staged through shared memory, whole columns per lane
   bool blocking_sync = false;     // host waits sleep on a blocking-sync event instead of spinning
   // when set (batched serving), the chain's FP64 products go through this call instead of their own
   // launch: it joins them to the products of other systems in one persistent launch
   std::function<void(ProductPlan&, double*, const double*, double*, int)> batch_submit;
   cudaEvent_t sync_ev = nullptr;
+  std::set<const void*> smem_allowed;   // kernels whose dynamic shared-memory limit was raised
   ProductProfile prof;
   ~System();
 };
@@ -337,6 +339,7 @@ void pinned_put(uint64_t* p);
 
 // index.cu
 void upload_geometry(System& S);
+int64_t dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st);   // out[0..n], returns the total
 void build_range_index(System& S, RangeIndex& R);
 ProductPlan& get_plan(System& S, int mult_type, int ra, int rb, int rc);
 AddMap& get_addmap(System& S, int ra, int rb);
@@ -355,7 +358,7 @@ struct BatchItem {                 // one FP64 product of a batched launch (role
   int exact;
 };
 void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st);
-void ensure_product_order(System& S, ProductPlan& P);   // the 4 x 4 kernels' output order (built once)
+void ensure_product_order(System& S, ProductPlan& P);   // the staged kernels' output order (built once)
 
 // gen.cu: synthetic S (which = 0) or H (which = 1) of range r into out
 void generate_SH(System& S, int r, int which, uint64_t seed, double* out);

@@ -413,6 +413,8 @@ int read_flag(int* d, cudaStream_t st) {
 
 }  // namespace
 
+int64_t dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st) { return exclusive_scan(in, n, out, st); }
+
 void upload_geometry(System& S) {
   Geometry& g = S.geo;
   DevGeometry& d = S.dg;

@@ -560,71 +560,6 @@ __global__ void __launch_bounds__(128, 8) k_mult_nd4_quad(MultArgs M, const int*
   }
 }
 
-// Any block sizes up to 16 (DZP 13 x 13, mixed SZ/DZP): one warp per output block, each lane a
-// 4 x 2 register tile of the output block (rows 4rt..4rt+3, columns 2ct..2ct+1, lane = rt * nct + ct),
-// so per term of the inner sum a lane loads 4 + 2 operand values for 8 multiply-adds instead of
-// 2 per multiply-add.  The order of the terms of every element is unchanged.
-template <int TYPE, bool EXACT>
-__device__ __forceinline__ void warp_tile(const MultArgs& M, int q) {
-  const int lane = threadIdx.x & 31;
-  const int ndi = M.prim_nsf[M.o_row[q]];
-  const int ndo = M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
-  const int nct = (ndo + 1) >> 1, nrt = (ndi + 3) >> 2;
-  const int rt = lane / nct, ct = lane - rt * nct;
-  const bool live = rt < nrt;                       // lanes beyond the tiles only keep the warp together
-  int r[4], c[2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) r[i] = min(4 * rt + i, ndi - 1);     // clamped: in-bounds reads
-#pragma unroll
-  for (int j = 0; j < 2; ++j) c[j] = min(2 * ct + j, ndo - 1);
-  double acc[4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { acc[i][0] = 0.0; acc[i][1] = 0.0; }
-  const int64_t p0 = M.ptr[q], p1 = M.ptr[q + 1];
-  if (live) {
-    for (int64_t t = p0; t < p1; ++t) {
-      const int2 pr = __ldcs(M.pairs + t);
-      const double* X = M.x + M.x_elem[pr.x];
-      const double* B = M.b + M.b_elem[pr.y];
-      if (TYPE == 1) {
-        const int ndk = M.cover_nsf[M.x_cover[pr.x]];
-        for (int n3 = 0; n3 < ndk; ++n3) {
-          double xv[4], bv[2];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) xv[i] = __ldg(X + r[i] + ndi * n3);
-#pragma unroll
-          for (int j = 0; j < 2; ++j) bv[j] = __ldg(B + n3 + ndk * c[j]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) acc[i][j] = madd<EXACT>(acc[i][j], xv[i], bv[j]);
-        }
-      } else {
-        const int ndj = M.cover_nsf[M.b_cover[pr.y]];
-        for (int n2 = 0; n2 < ndj; ++n2) {
-          double xv[4], bv[2];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) xv[i] = __ldg(X + r[i] + ndi * n2);
-#pragma unroll
-          for (int j = 0; j < 2; ++j) bv[j] = __ldg(B + c[j] + ndo * n2);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) acc[i][j] = madd<EXACT>(acc[i][j], xv[i], bv[j]);
-        }
-      }
-    }
-    double* O = M.out + M.o_elem[q];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int n1 = 4 * rt + i, n2 = 2 * ct + j;
-        if (n1 < ndi && n2 < ndo) O[n1 + ndi * n2] = acc[i][j];
-      }
-  }
-}
-
 // FP64 on the tensor cores (DMMA, mma.sync.m8n8k4.f64): one warp per output block, the block padded to
 // 16 x 16 as 2 x 2 tiles of 8 x 8, the contraction in steps of 4.  Per step a lane loads one element of
 // each first-operand row tile (row g = lane / 4, column t = lane % 4 of the step) and one of each B column
@@ -715,24 +650,244 @@ __global__ void __launch_bounds__(128) k_mult_dmma(MultArgs M) {
       }
 }
 
-template <int TYPE, bool EXACT>
-__global__ void __launch_bounds__(256) k_mult_tile(MultArgs M) {
-  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= M.n_out) return;
-  warp_tile<TYPE, EXACT>(M, q);
+// Any block sizes up to 16 (DZP 13 x 13, mixed SZ/DZP): LPB lanes per output block (8: four blocks per warp,
+// lane l owns columns l and l + 8; 16: two blocks per warp, one column per lane), every row of those columns in
+// the lane's registers.  The group stages the two operand blocks of a pair in shared memory with cp.async; X
+// with its columns padded to an even length, so that two row values are one 16-byte read that all lanes of a
+// group share, B in its stored layout (a block of odd size starts on an 8-byte boundary: its copy keeps the
+// source's 8-byte phase and moves the odd first or last element alone).  Buffers are an odd multiple of 32
+// bytes long, so the groups' broadcast reads fall into different banks.  The order of the terms of every
+// element is unchanged.
+//
+// What bounds it: the FP64 pipe and the shared-memory reads.  A 13 x 13 pair is 2 x 13^3 FP64 instructions on
+// 13 of 16 columns (84 SM cycles); a 16-byte read takes two L1 wavefronts even as a broadcast, so with LPB = 8 a
+// pair costs about 88 wavefronts, with LPB = 16 129.  Against it LPB = 8 needs twice the shared memory per warp.
+// Measured (64-atom DZP cell, LS.L -> LSL, 147794 output blocks, 4.2 M pairs, reference rounding; TFLOP/s): LPB 8
+// with one stage 10.5, with two 9.7 and three 9.1 (fewer warps per SM); LPB 16 with one 9.3, two 9.2, four 7.9;
+// one block per warp with 4 x 2 tiles and operands read from global memory 3.4.  With many warps per SM the
+// other warps hide a stage's latency, so one stage is best.  With few output blocks (3008, type 2 into the H
+// range) LPB 16 with two stages runs at 7.4 against 6.2: twice the warps, and the next pair's copies in flight.
+// The two are equal near 8000 output blocks (8.6).
+// U: the block size when the whole system has one, else 0.  MAXND: no block is larger.
+template <int MAXND, int LPB, int STAGES>
+struct GroupShape {
+  static constexpr int kBlocks = 32 / LPB;                            // output blocks per warp
+  // bytes of one staged block, odd multiples of 32: X with its columns padded to an even length, B as stored
+  static constexpr int kStrideX = 32 * (((MAXND + 1) / 2 * 2 * MAXND * 8 + 31) / 32 | 1);
+  static constexpr int kStrideB = 32 * ((MAXND * MAXND * 8 + 8 + 31) / 32 | 1);
+  static constexpr int kStage = kBlocks * (kStrideX + kStrideB);      // the X blocks, then the B blocks
+  static constexpr int kWarpBytes = STAGES * kStage;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+
+// n doubles at src (8-byte aligned) to the 16-byte aligned slot dst, by the LPB lanes l of a group; the data
+// starts at dst + 8 when src is not 16-byte aligned.  Reads no byte outside [src, src + n).
+template <int U, int LPB>
+__device__ __forceinline__ void group_copy(uint32_t dst, const double* src, int n, int l) {
+  const int sh = (int)(((uintptr_t)src >> 3) & 1);
+  const int chunks = (n - sh) >> 1;
+  const double* s16 = src + sh;
+  const uint32_t d16 = dst + 16 * sh;
+  if constexpr (U > 0) {
+    constexpr int kIter = (U * U / 2 + LPB - 1) / LPB;
+#pragma unroll
+    for (int v = 0; v < kIter; ++v)
+      if (l + LPB * v < chunks) cp_async16(d16 + 16 * (l + LPB * v), s16 + 2 * (l + LPB * v));
+  } else {
+    for (int v = l; v < chunks; v += LPB) cp_async16(d16 + 16 * v, s16 + 2 * v);
+  }
+  if (l == LPB - 2 && sh) cp_async8(dst + 8, src);
+  if (l == LPB - 1 && ((n - sh) & 1)) cp_async8(dst + 8 * (sh + n - 1), src + n - 1);
+}
+
+// The X block (rows x cols, n = rows * cols doubles at src) to the slot dst with its columns ld doubles apart
+// (rows rounded up to even), so that two row values are one 16-byte shared-memory read.  magic: 65536 / rows + 1.
+template <int U, int LPB>
+__device__ __forceinline__ void group_copy_columns(uint32_t dst, const double* src, int n, int rows, int magic, int l) {
+  if constexpr (U > 0) {
+    constexpr int kIter = (U * U + LPB - 1) / LPB;
+#pragma unroll
+    for (int v = 0; v < kIter; ++v) {
+      const int e = l + LPB * v;
+      if (e < U * U) cp_async8(dst + 8 * (e + (U & 1) * (e / U)), src + e);
+    }
+  } else {
+    const int pad = rows & 1;
+    for (int e = l; e < n; e += LPB) cp_async8(dst + 8 * (e + pad * ((e * magic) >> 16)), src + e);
+  }
+}
+
+// One pair's arithmetic: acc[r][h] (row r, column c[h]) += sum over n < nk.
+template <int TYPE, bool EXACT, int U, int R, bool FULL, int H>
+__device__ __forceinline__ void group_compute(const double2* __restrict__ X, const double* __restrict__ B, int ndi, int ndo,
+                                              int nk, const int (&c)[H], int cols, double (&acc)[R][H]) {
+  const int half = FULL ? (R + 1) / 2 : (ndi + 1) >> 1;           // double2 per column of X
+  auto step = [&](int n) {
+    double2 x[(R + 1) / 2];
+    double b[H];
+#pragma unroll
+    for (int r = 0; r < (R + 1) / 2; ++r) x[r] = X[(FULL ? r : min(r, half - 1)) + half * n];
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      if (h < cols) b[h] = TYPE == 1 ? B[n + nk * c[h]] : B[c[h] + ndo * n];
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      if (h < cols) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r][h] = madd<EXACT>(acc[r][h], r & 1 ? x[r / 2].y : x[r / 2].x, b[h]);
+      }
+  };
+  if constexpr (U > 0) {
+#pragma unroll
+    for (int n = 0; n < U; ++n) step(n);
+  } else {
+#pragma unroll 2
+    for (int n = 0; n < nk; ++n) step(n);
+  }
+}
+
+// One warp: output slots [base, base + 32 / LPB) of `order`; W: this warp's shared memory (STAGES stages).
+// R: rows of the register tile; FULL: every block of the warp has exactly R rows.
+template <int TYPE, bool EXACT, int U, int MAXND, int LPB, int STAGES, int R, bool FULL>
+__device__ __forceinline__ void warp_group_rows(const MultArgs& M, const int* __restrict__ order, int base, unsigned char* W) {
+  using Q = GroupShape<MAXND, LPB, STAGES>;
+  constexpr int H = 16 / LPB;                      // columns per lane
+  const unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31, g = lane / LPB, l = lane % LPB;
+  const bool has = base + g < M.n_out;
+  const int q = has ? order[base + g] : 0;
+  const int ndi = FULL ? R : M.prim_nsf[M.o_row[q]];
+  const int ndo = U > 0 ? U : M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
+  int c[H];
+#pragma unroll
+  for (int h = 0; h < H; ++h) c[h] = min(l + LPB * h, ndo - 1);   // clamped: in-bounds reads
+  const int cols = H == 1 || (U > 0 ? U > LPB : __any_sync(kFull, ndo > LPB)) ? H : 1;
+  const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
+  const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;       // a list is no longer than a row: fits 32 bits
+  const int steps = __reduce_max_sync(kFull, nt);
+  double acc[R][H];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int h = 0; h < H; ++h) acc[r][h] = 0.0;
+  const uint32_t w0 = smem_addr(W);
+  const int magic = U > 0 ? 0 : 65536 / ndi + 1;   // e / ndi = e * magic >> 16 for e < 256, ndi <= 16
+  // operand addresses and inner dimension of a pair; looked up one step before its copies are issued
+  struct Term { const double *x, *b; int nk; };
+  auto look_up = [&](int2 pr) {
+    Term v;
+    v.x = M.x + (U > 0 ? (int64_t)pr.x * (U * U) : M.x_elem[pr.x]);
+    v.b = M.b + (U > 0 ? (int64_t)pr.y * (U * U) : M.b_elem[pr.y]);
+    v.nk = U > 0 ? U : (TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]]);
+    return v;
+  };
+  Term next = {nullptr, nullptr, 0};               // pair `issued`
+  int2 pn = make_int2(0, 0);                       // pair `issued + 1`
+  if (nt > 0) next = look_up(__ldcs(pairs));
+  if (nt > 1) pn = __ldcs(pairs + 1);
+  int issued = 0, slot = 0;                        // pairs whose copies were issued, and the stage of the next one
+  int meta[STAGES];                                // 2 nk + the 8-byte phase of the B copy, per stage in flight
+  auto issue = [&]() {
+    int mt = 0;
+    if (issued < nt) {
+      const uint32_t d = w0 + slot * Q::kStage;
+      mt = 2 * next.nk + (int)(((uintptr_t)next.b >> 3) & 1);
+      group_copy_columns<U, LPB>(d + g * Q::kStrideX, next.x, ndi * next.nk, ndi, magic, l);
+      group_copy<U, LPB>(d + Q::kBlocks * Q::kStrideX + g * Q::kStrideB, next.b, next.nk * ndo, l);
+      if (issued + 1 < nt) next = look_up(pn);
+      if (issued + 2 < nt) pn = __ldcs(pairs + issued + 2);
+    }
+    cp_async_commit();
+    ++issued;
+    slot = slot + 1 == STAGES ? 0 : slot + 1;
+#pragma unroll
+    for (int k = 0; k + 1 < STAGES; ++k) meta[k] = meta[k + 1];
+    meta[STAGES - 1] = mt;
+  };
+#pragma unroll
+  for (int k = 0; k < STAGES; ++k) meta[k] = 0;
+#pragma unroll
+  for (int k = 0; k + 1 < STAGES; ++k) issue();
+  int st = 0;
+  for (int t = 0; t < steps; ++t) {
+    issue();
+    cp_async_wait<STAGES - 1>();
+    __syncwarp();
+    if (t < nt) {
+      const unsigned char* s = W + st * Q::kStage;
+      const double2* X = reinterpret_cast<const double2*>(s + g * Q::kStrideX);
+      const double* B = reinterpret_cast<const double*>(s + Q::kBlocks * Q::kStrideX + g * Q::kStrideB) + (meta[0] & 1);
+      group_compute<TYPE, EXACT, U, R, FULL, H>(X, B, ndi, ndo, meta[0] >> 1, c, cols, acc);
+    }
+    __syncwarp();                                  // the stage is read before the next issue() refills it
+    st = st + 1 == STAGES ? 0 : st + 1;
+  }
+  // results through shared memory (the staging buffers are free: no copy is in flight), so that a group
+  // writes its block to consecutive addresses
+  double* O = reinterpret_cast<double*>(W + g * Q::kStrideX);
+#pragma unroll
+  for (int h = 0; h < H; ++h)
+    if (l + LPB * h < ndo) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (FULL || r < ndi) O[r + ndi * (l + LPB * h)] = acc[r][h];
+    }
+  __syncwarp();
+  if (has) {
+    double* D = M.out + (U > 0 ? (int64_t)q * (U * U) : M.o_elem[q]);
+    for (int e = l; e < ndi * ndo; e += LPB) __stcs(D + e, O[e]);
+  }
+  __syncwarp();
+}
+
+template <int TYPE, bool EXACT, int U, int MAXND, int LPB, int STAGES>
+__device__ __forceinline__ void warp_group(const MultArgs& M, const int* __restrict__ order, int base, unsigned char* W) {
+  if constexpr (U > 0) {
+    warp_group_rows<TYPE, EXACT, U, MAXND, LPB, STAGES, U, true>(M, order, base, W);
+  } else {
+    // several sizes: a warp whose blocks all have four rows, or all MAXND, runs a tile of exactly that height
+    // (the order keeps blocks of one row count together)
+    const int s = min(base + (threadIdx.x & 31) / LPB, M.n_out - 1);
+    const int ndi = M.prim_nsf[M.o_row[order[s]]];
+    if (__all_sync(0xffffffffu, ndi == 4)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, 4, true>(M, order, base, W);
+    else if (__all_sync(0xffffffffu, ndi == MAXND)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, true>(M, order, base, W);
+    else warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, false>(M, order, base, W);
+  }
+}
+
+template <int TYPE, bool EXACT, int U, int MAXND, int LPB, int STAGES>
+__global__ void __launch_bounds__(64) k_mult_group(MultArgs M, const int* __restrict__ order) {
+  extern __shared__ __align__(128) unsigned char group_smem[];
+  using Q = GroupShape<MAXND, LPB, STAGES>;
+  const int warp = threadIdx.x >> 5;
+  const int base = (blockIdx.x * 2 + warp) * Q::kBlocks;
+  if (base >= M.n_out) return;                  // whole warp
+  warp_group<TYPE, EXACT, U, MAXND, LPB, STAGES>(M, order, base, group_smem + warp * Q::kWarpBytes);
 }
 
 // Many independent products in one persistent launch (the concatenation of their output-block
 // lists): every warp takes work units u = warp id, warp id + warps in the grid, ...; a unit is 32
-// output slots of a uniform 4 x 4 product (the warp-staged kernel) or one output block of any other
-// product (the register-tiled kernel).  Each output block is computed by exactly the operations of the
-// single-product kernels, so the results are the same bits as separate launches.  The product table
-// travels in the kernel's parameters (no host-to-device copy before the launch).
+// output slots of a uniform 4 x 4 product (the warp-staged kernel) or two output blocks of any other
+// product (the group kernel with 16 lanes per block).  Each output block is computed by exactly the operations
+// of the single-product kernels, so the results are the same bits as separate launches.  The product table
+// travels in the kernel's parameters (no host-to-device copy before the launch).  Eight systems of 64 to 300 atoms
+// (1.98 GFLOP): 0.284 ms, against 0.684 ms with one output block per warp and register tiles of 4 x 2.
 struct BatchProduct {
   MultArgs M;
-  const int* order;                // 4 x 4 products: output blocks by descending pair count
-  int kind;                        // bit 0: type 2, bit 1: exact rounding, bit 2: uniform 4 x 4 blocks
+  const int* order;                // output blocks by descending pair count
+  int kind;                        // bit 0: type 2, bit 1: exact rounding, bits 2..: kBatchNd4, ...
 };
+enum { kBatchNd4 = 0, kBatchU13 = 4, kBatchMax13 = 8, kBatchMax16 = 12 };
 constexpr int kBatchMax = 96;      // products per launch (the table stays within the 32 KB parameter space)
 struct BatchParams {
   int n_prod;
@@ -741,9 +896,26 @@ struct BatchParams {
 };
 static_assert(sizeof(BatchParams) < 32000, "batched product table exceeds the kernel parameter space");
 
-__global__ void __launch_bounds__(128, 5) k_mult_batch(const __grid_constant__ BatchParams B) {
-  __shared__ double2 sx[4][32 * kStageStride];
-  __shared__ double2 sb[4][32 * kStageStride];
+constexpr int kBatchWarpBytes = 2 * 32 * kStageStride * 16;    // the warp-staged 4 x 4 kernel's X and B
+static_assert(GroupShape<13, 16, 1>::kWarpBytes <= kBatchWarpBytes && GroupShape<16, 16, 1>::kWarpBytes <= kBatchWarpBytes,
+              "batched warps share one staging area");
+
+template <int TYPE, bool EXACT>
+__device__ __forceinline__ void batch_unit(const BatchProduct& P, int family, int unit, unsigned char* W) {
+  if (family == kBatchNd4) {
+    double2* X = reinterpret_cast<double2*>(W);
+    warp_nd4_staged<TYPE, EXACT>(P.M, P.order, unit * 32, X, X + 32 * kStageStride);
+  } else if (family == kBatchU13) {
+    warp_group<TYPE, EXACT, 13, 13, 16, 1>(P.M, P.order, unit * 2, W);
+  } else if (family == kBatchMax13) {
+    warp_group<TYPE, EXACT, 0, 13, 16, 1>(P.M, P.order, unit * 2, W);
+  } else {
+    warp_group<TYPE, EXACT, 0, 16, 16, 1>(P.M, P.order, unit * 2, W);
+  }
+}
+
+__global__ void __launch_bounds__(128, 4) k_mult_batch(const __grid_constant__ BatchParams B) {
+  __shared__ __align__(128) unsigned char smem[4][kBatchWarpBytes];
   const int warp = threadIdx.x >> 5;
   const int n_units = B.unit_off[B.n_prod];
   for (int u = blockIdx.x * 4 + warp; u < n_units; u += gridDim.x * 4) {
@@ -753,18 +925,14 @@ __global__ void __launch_bounds__(128, 5) k_mult_batch(const __grid_constant__ B
       if (B.unit_off[mid] <= u) lo = mid; else hi = mid - 1;
     }
     const BatchProduct& P = B.prods[lo];
-    const int kind = P.kind;
-    const int first = (u - B.unit_off[lo]) * ((kind & 4) ? 32 : 1);
-    switch (kind) {
-      case 0: warp_tile<1, false>(P.M, first); break;
-      case 1: warp_tile<2, false>(P.M, first); break;
-      case 2: warp_tile<1, true>(P.M, first); break;
-      case 3: warp_tile<2, true>(P.M, first); break;
-      case 4: warp_nd4_staged<1, false>(P.M, P.order, first, sx[warp], sb[warp]); break;
-      case 5: warp_nd4_staged<2, false>(P.M, P.order, first, sx[warp], sb[warp]); break;
-      case 6: warp_nd4_staged<1, true>(P.M, P.order, first, sx[warp], sb[warp]); break;
-      default: warp_nd4_staged<2, true>(P.M, P.order, first, sx[warp], sb[warp]); break;
+    const int family = P.kind & ~3, unit = u - B.unit_off[lo];
+    switch (P.kind & 3) {
+      case 0: batch_unit<1, false>(P, family, unit, smem[warp]); break;
+      case 1: batch_unit<2, false>(P, family, unit, smem[warp]); break;
+      case 2: batch_unit<1, true>(P, family, unit, smem[warp]); break;
+      default: batch_unit<2, true>(P, family, unit, smem[warp]); break;
     }
+    __syncwarp();                                // the staging area goes to the next unit
   }
 }
 
@@ -812,15 +980,84 @@ void launch_dropin(int type, const int64_t* d_out, const int* d_dims, const int6
   CQ_CUDA(cudaGetLastError());
 }
 
-// output blocks by descending pair count (stable): lanes of a warp get similar list lengths
+// Output blocks by descending pair count (blocks of more than four rows first in systems of several sizes):
+// the lanes of a warp get lists of similar length and the long ones start first.  A stable counting sort on the
+// device (blocks of equal count keep their order: neighbours in a row share operand blocks in the caches).
+namespace {
+constexpr int kOrderTile = 1024;      // blocks counted and placed by one CTA
+
+struct OrderKey {
+  const int64_t* ptr;
+  const int *o_row, *prim_nsf;
+  int by_rows, counts;                // counts: bins per row class
+  __device__ __forceinline__ int operator()(int q) const {
+    const int c = (int)min(ptr[q + 1] - ptr[q], (int64_t)(counts - 1));
+    return (by_rows && prim_nsf[o_row[q]] <= 4 ? counts : 0) + counts - 1 - c;
+  }
+};
+// hist[bin * tiles + tile]: blocks of the tile in the bin
+__global__ void __launch_bounds__(256) k_order_count(OrderKey key, int n, int bins, int* __restrict__ hist) {
+  extern __shared__ int order_bins[];
+  for (int b = threadIdx.x; b < bins; b += 256) order_bins[b] = 0;
+  __syncthreads();
+  for (int q = blockIdx.x * kOrderTile + threadIdx.x; q < min(n, (int)(blockIdx.x + 1) * kOrderTile); q += 256)
+    atomicAdd(order_bins + key(q), 1);
+  __syncthreads();
+  for (int b = threadIdx.x; b < bins; b += 256) hist[(size_t)b * gridDim.x + blockIdx.x] = order_bins[b];
+}
+// first: the exclusive scan of hist.  The warps of a CTA place their 32 blocks one after the other.
+__global__ void __launch_bounds__(256) k_order_fill(OrderKey key, int n, int bins, const int64_t* __restrict__ first,
+                                                    int* __restrict__ order) {
+  extern __shared__ int order_bins[];
+  for (int b = threadIdx.x; b < bins; b += 256) order_bins[b] = (int)first[(size_t)b * gridDim.x + blockIdx.x];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int q0 = blockIdx.x * kOrderTile; q0 < min(n, (int)(blockIdx.x + 1) * kOrderTile); q0 += 256) {
+    const int q = q0 + threadIdx.x, bin = q < n ? key(q) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    const int lead = __ffs(peers) - 1;
+    for (int w = 0; w < 8; ++w) {
+      __syncthreads();
+      if (w != warp) continue;
+      int at = 0;
+      if (bin >= 0 && lane == lead) { at = order_bins[bin]; order_bins[bin] = at + __popc(peers); }
+      at = __shfl_sync(0xffffffffu, at, lead);
+      if (bin >= 0) order[at + __popc(peers & ((1u << lane) - 1u))] = q;
+    }
+  }
+}
+}  // namespace
+
 static void ensure_order(System& S, ProductPlan& P) {
-  if (P.order.n != 0) return;
-  std::vector<int64_t> ptr = P.ptr.download(S.stream);
-  const int n_out = (int)ptr.size() - 1;
-  std::vector<int> ord(std::max(n_out, 0));
-  std::iota(ord.begin(), ord.end(), 0);
-  std::stable_sort(ord.begin(), ord.end(), [&](int u, int v) { return ptr[u + 1] - ptr[u] > ptr[v + 1] - ptr[v]; });
-  P.order.upload(ord, S.stream);
+  const RangeIndex& O = *S.ranges[P.out_range];
+  if (P.order.n != 0 || O.nnz == 0) return;
+  OrderKey key;
+  key.ptr = P.ptr.p;
+  key.o_row = O.nb_row.p;
+  key.prim_nsf = S.dg.prim_nsf.p;
+  key.by_rows = S.uniform_nsf == 0;
+  // a pair list is no longer than a row of either operand; counts above 4095 share a bin
+  const int longest = std::min(S.ranges[P.mult_type == 1 ? P.ra : P.rc]->max_row, S.ranges[P.rb]->max_row);
+  key.counts = std::min(longest, 4095) + 1;
+  const int bins = key.counts * (key.by_rows ? 2 : 1), tiles = (O.nnz + kOrderTile - 1) / kOrderTile;
+  DevBuf<int> hist;
+  DevBuf<int64_t> first;
+  hist.alloc((size_t)bins * tiles, S.stream);
+  first.alloc((size_t)bins * tiles + 1, S.stream);
+  k_order_count<<<tiles, 256, bins * sizeof(int), S.stream>>>(key, O.nnz, bins, hist.p);
+  CQ_CUDA(cudaGetLastError());
+  dev_exclusive_scan(hist.p, (int64_t)bins * tiles, first.p, S.stream);
+  P.order.alloc(O.nnz, S.stream);
+  k_order_fill<<<tiles, 256, bins * sizeof(int), S.stream>>>(key, O.nnz, bins, first.p, P.order.p);
+  S.launches += 2;
+  CQ_CUDA(cudaGetLastError());
+}
+
+// Dynamic shared memory above 48 KB has to be allowed per kernel (once per system and kernel).
+template <class K>
+static void allow_smem(System& S, K* kern, int bytes) {
+  const void* k = reinterpret_cast<const void*>(kern);
+  if (!S.smem_allowed.insert(k).second) return;
+  CQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
 // One launch of the FP64 product with kernel `variant` (0..3 and 5 for uniform 4 x 4 blocks with
@@ -837,7 +1074,7 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
     int* err = device_timeout_word(S);
     auto launch = [&](auto kern) {
-      CQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(S, kern, (int)smem);
       kern<<<grid, 128, smem, st>>>(M, P.order.p, err);
     };
     if (P.mult_type == 1) {
@@ -897,11 +1134,29 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) k_mult_nd4<2, true><<<grid, T, 0, st>>>(M); else k_mult_nd4<2, false><<<grid, T, 0, st>>>(M);
     }
   } else if (variant == 4) {
-    int grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
+    ensure_order(S, P);
+    auto launch = [&](auto kern, int blocks, int warp_bytes) {
+      allow_smem(S, kern, 2 * warp_bytes);
+      kern<<<(M.n_out + 2 * blocks - 1) / (2 * blocks), 64, 2 * warp_bytes, st>>>(M, P.order.p);
+    };
+    auto by_size = [&](auto type, auto ex) {
+      constexpr int TY = decltype(type)::value;
+      constexpr bool EX = decltype(ex)::value;
+      auto by_group = [&](auto lpb, auto stages) {
+        constexpr int LPB = decltype(lpb)::value, ST = decltype(stages)::value;
+        if (S.uniform_nsf == 13) launch(k_mult_group<TY, EX, 13, 13, LPB, ST>, 32 / LPB, GroupShape<13, LPB, ST>::kWarpBytes);
+        else if (S.max_nsf <= 13) launch(k_mult_group<TY, EX, 0, 13, LPB, ST>, 32 / LPB, GroupShape<13, LPB, ST>::kWarpBytes);
+        else launch(k_mult_group<TY, EX, 0, 16, LPB, ST>, 32 / LPB, GroupShape<16, LPB, ST>::kWarpBytes);
+      };
+      // four blocks per warp once they give every SM its 18 resident warps (see k_mult_group)
+      if (M.n_out >= 148 * 18 * 4) by_group(std::integral_constant<int, 8>{}, std::integral_constant<int, 1>{});
+      else by_group(std::integral_constant<int, 16>{}, std::integral_constant<int, 2>{});
+    };
+    using std::integral_constant;
     if (P.mult_type == 1) {
-      if (exact) k_mult_tile<1, true><<<grid, T, 0, st>>>(M); else k_mult_tile<1, false><<<grid, T, 0, st>>>(M);
+      if (exact) by_size(integral_constant<int, 1>{}, std::true_type{}); else by_size(integral_constant<int, 1>{}, std::false_type{});
     } else {
-      if (exact) k_mult_tile<2, true><<<grid, T, 0, st>>>(M); else k_mult_tile<2, false><<<grid, T, 0, st>>>(M);
+      if (exact) by_size(integral_constant<int, 2>{}, std::true_type{}); else by_size(integral_constant<int, 2>{}, std::false_type{});
     }
   } else {
     int grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
@@ -922,16 +1177,18 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
 // bits and each fully overwrites the output, so tuning changes speed only; the last timed launch
 // leaves the correct result.
 static int tuned_variant(System& S, ProductPlan& P, const MultArgs& M, int exact, bool nd4) {
+  if (!nd4) {                      // untimed: the generic kernel is 3 to 5 times slower on every product
+    if (S.uniform_nsf != 4) P.tuned = 4;
+    return 4;
+  }
   if (P.tuned >= 0) return P.tuned;
-  // candidates, the preferred kernel first: uniform 4x4 blocks: warp-staged, four lanes per
+  // candidates of uniform 4x4 blocks, the preferred kernel first: warp-staged, four lanes per
   // block, thread per block, 16 lanes per block (the last two the most parallel, for products with
-  // few output blocks); other sizes: register-tiled, generic
+  // few output blocks)
   // (variant 6, the bulk-copy-staged kernel, is not a candidate: 2.4x slower than variant 3 on every
   // product of the 512-atom SZ chain, since one 128-byte bulk copy takes about 11 SM cycles)
-  int cands[4];
-  int nc = 0;
-  if (nd4) { cands[0] = 3; cands[1] = 5; cands[2] = 1; cands[3] = 0; nc = 4; }
-  else { cands[0] = 4; cands[1] = 0; nc = 2; }
+  const int cands[4] = {3, 5, 1, 0};
+  const int nc = 4;
   cudaEvent_t e0, e1;
   CQ_CUDA(cudaEventCreate(&e0));
   CQ_CUDA(cudaEventCreate(&e1));
@@ -1013,9 +1270,7 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   }
 }
 
-void ensure_product_order(System& S, ProductPlan& P) {
-  if (S.uniform_nsf == 4) ensure_order(S, P);
-}
+void ensure_product_order(System& S, ProductPlan& P) { ensure_order(S, P); }
 
 // Products of independent systems (or of one system) in persistent launches on `st` (up to kBatchMax
 // products each).  The caller orders `st` after the work the operands depend on and the systems' later
@@ -1044,12 +1299,13 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
     BatchProduct bp;
     bp.M = product_args(S, P, it.a, it.b, it.c, &nd4);
     if (bp.M.n_out == 0) continue;
-    if (nd4) ensure_order(S, P);
-    bp.order = nd4 ? P.order.p : nullptr;
-    bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) | (nd4 ? 4 : 0);
+    CQ_CHECK(P.order.p != nullptr, CQ_ERR_STATE, "batched product without its output order (ensure_product_order)");
+    bp.order = P.order.p;
+    bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) |
+              (nd4 ? kBatchNd4 : S.uniform_nsf == 13 ? kBatchU13 : S.max_nsf <= 13 ? kBatchMax13 : kBatchMax16);
     if (B.n_prod == kBatchMax) { flush(); B.unit_off[0] = 0; }
     B.prods[B.n_prod] = bp;
-    B.unit_off[B.n_prod + 1] = B.unit_off[B.n_prod] + (nd4 ? (bp.M.n_out + 31) / 32 : bp.M.n_out);
+    B.unit_off[B.n_prod + 1] = B.unit_off[B.n_prod] + (nd4 ? (bp.M.n_out + 31) / 32 : (bp.M.n_out + 1) / 2);
     ++B.n_prod;
     S.launches++;
   }

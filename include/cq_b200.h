@@ -276,9 +276,9 @@ int cq_generate_SH(cq_system* sys, int r, int which, uint64_t seed, double* out)
  * memory, 5 = four lanes per output block (one column each), the first operand's block staged
  * in shared memory, 6 = one thread per output block with its operand blocks staged by bulk copies
  * (cp.async.bulk, completion on an mbarrier, bounded waits); for other block sizes (DZP 13 x 13,
- * mixed sizes) 0 = one warp per output block, one lane per element, 4 = one warp per output block,
- * a 4 x 2 register tile per lane (the autotuner candidates are 3/5/1/0 for uniform 4 x 4 blocks
- * and 4/0 otherwise; variant 6 is selectable only).  All give
+ * mixed sizes) 0 = one warp per output block, one lane per element, 4 = two or four output blocks per
+ * warp, their operand blocks staged in shared memory, whole columns per lane (the autotuner candidates are
+ * 3/5/1/0 for uniform 4 x 4 blocks, and 4 is used untimed otherwise; variant 6 is selectable only).  All give
  * identical results.
  * CQ_OPT_BLOCKING_SYNC: 1 = the host thread sleeps on a blocking-sync event whenever the
  * solver waits for a scalar from the device (many concurrent solvers per host core), 0 = it
