@@ -293,7 +293,7 @@ class System:
         return t.value, f.value
 
     def product_tuning(self, mult_type, ra, rb, rc, mixed=False):
-        """FP64: (variant chosen by the autotuner or -1, {variant: timed ms}); mixed=True: (output blocks per
+        """FP64: (variant chosen by the rule on sizes or -1, {variant: timed ms}); mixed=True: (output blocks per
         warp chosen for the split-precision kernel or -1, {group size: timed ms})."""
         v, g = c_int(), c_int()
         ms, gms = (ctypes.c_float * 7)(), (ctypes.c_float * 4)()
@@ -347,7 +347,7 @@ class System:
         check(lib().cq_system_set_stream(self._h, c_void_p(stream) if stream else None))
 
     def set_mult_variant(self, v):
-        """FP64 4x4 product kernel: -1 = autotuned per product (default), 0 = one lane per output element,
+        """FP64 4x4 product kernel: -1 = chosen per product by size (default), 0 = one lane per output element,
         1 = one thread per output block, 2 = operand row staged in shared memory, 3 = warp-staged operand blocks,
         5 = four lanes per output block, 6 = operand blocks staged by bulk copies."""
         check(lib().cq_system_set_option(self._h, 1, int(v)))

@@ -207,8 +207,10 @@ struct ProductPlan {
   DevBuf<int2> pairs;             // [n_pairs] (x block, b block)
   int n_tiles = 0;                // row tiles of the staged 4x4 kernel: (q0, q1, x row first, x row end)
   DevBuf<int4> tiles;
+  int n_row_tiles = -1;           // tiles of the type-2 4x4 row kernel: (B row first, end, trans_dest first, outputs)
+  DevBuf<int4> row_tiles;
   DevBuf<int> order;              // output blocks by descending pair count (staged kernels)
-  int tuned = -1;                 // FP64 kernel variant chosen by the autotuner (-1: not tuned yet)
+  int tuned = -1;                 // FP64 kernel variant chosen by auto_variant (-1: not chosen yet)
   float tune_ms[7] = {0, 0, 0, 0, 0, 0, 0};
 };
 
@@ -314,11 +316,11 @@ struct System {
   DevBuf<double> diag_buf;        // gathered onsite diagonal (exact trace)
   uint64_t* host_res = nullptr;   // pinned host copy of the exact-sum results (4 words per sum)
   int64_t launches = 0;           // kernels launched by this system (all kinds)
-  int mult_variant = -1;          // 4x4 FP64 product kernel: -1 = chosen per product by the autotuner,
+  int mult_variant = -1;          // 4x4 FP64 product kernel: -1 = chosen per product by its sizes,
                                   // 0 = one lane per element, 1 = one thread per block,
                                   // 2 = one thread per block with the operand row staged in shared memory,
                                   // 3 = one thread per block with warp-cooperative staging of the operand blocks,
-                                  // 5 = four lanes per block, 6 = one thread per block with bulk-copy staging;
+                                  // 4 = type 2: 3 with a shared row of B, 5 = four lanes per block, 6 = one thread per block with bulk-copy staging;
                                   // other block sizes: 0 = generic warp per block, 4 = two or four blocks per
                                   // warp staged through shared memory, whole columns per lane
   bool blocking_sync = false;     // host waits sleep on a blocking-sync event instead of spinning

@@ -257,81 +257,98 @@ __global__ void __launch_bounds__(128) k_mult_nd4_rows(MultArgs M, const int4* _
   }
 }
 
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // 4 x 4 blocks, one thread per output block, operand blocks staged through shared memory by
-// the whole warp.  A thread-per-block kernel that reads its own operand blocks issues 16-byte
-// loads that touch 32 different blocks per warp instruction, which saturates the L1 on
-// wavefronts long before the FP64 pipe is busy.  Here, per step, the warp first copies the 32
-// (x, b) block pairs its lanes need with loads in which 8 consecutive lanes read one whole
-// 128-byte block (4 blocks per instruction), stores them in padded shared memory (9 x 16 bytes
-// per block: conflict-free 16-byte reads per quarter warp), then every lane does its own 4 x 4
-// product in the reference order.  Output blocks are taken in `order` (descending pair count)
-// so the lanes of a warp have pair lists of similar length.
-constexpr int kStageStride = 9;   // double2 per staged 4 x 4 block (8 + 1 padding)
+// the whole warp.  A thread-per-block kernel that reads its own operand blocks issues 16-byte loads that touch 32
+// different blocks per warp instruction, which saturates the L1 on wavefronts long before the FP64 pipe is busy.
+// Here, per step, the warp copies the 32 (x, b) block pairs its lanes need with cp.async (8 consecutive lanes move
+// one whole 128-byte block, 4 blocks per instruction), then every lane reads its two blocks and does its own
+// 4 x 4 product in the reference order.  Output blocks are taken in `order` (descending pair count) so the lanes
+// of a warp have pair lists of similar length.
+// What bounds it: the 256 bytes that a pair moves from L2 (49 of the 64 bytes per SM and cycle) and about four L1
+// wavefronts per pair.  The copies bypass the L1 (.cg): through it (.ca, or loads and shared-memory stores) the
+// same kernel spends six.  Measured on LS.L -> LSL of the 512-atom cell (34.0 M pairs): 0.566 ms with .cg, 0.901
+// with .ca, 1.009 with loads and stores; on the eight products of the LNV call 2.56, 3.96 and 4.58 ms.  One stage:
+// the other 19 warps of an SM hide its latency, and a second stage (0.578 ms) costs L1, which the pair lists use
+// (reading them two pairs at a time without it: 0.632 ms).
+constexpr int kStageBytes = 64 * 128;    // one step of a warp: 32 X and 32 B blocks
+
+// acc += the 4 x 4 product of the staged blocks x and b (both in registers), terms in the reference's order
+template <int TYPE, bool EXACT>
+__device__ __forceinline__ void nd4_mul_add(double (&acc)[16], const double (&x)[16], const double (&b)[16]) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n1 = 0; n1 < 4; ++n1) {
+      double a = acc[n1 + 4 * m];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) a = madd<EXACT>(a, x[n1 + 4 * n], TYPE == 1 ? b[n + 4 * m] : b[m + 4 * n]);
+      acc[n1 + 4 * m] = a;
+    }
+}
+// block `lane` of a stage: its 16-byte chunk v lies at chunk v ^ (lane & 7), so that the reads of eight lanes
+// fall into different banks
+__device__ __forceinline__ void nd4_read(double (&v)[16], const unsigned char* stage, int lane) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double2 d = *reinterpret_cast<const double2*>(stage + lane * 128 + ((k ^ (lane & 7)) << 4));
+    v[2 * k] = d.x; v[2 * k + 1] = d.y;
+  }
+}
 
 // One warp of the warp-staged 4 x 4 kernel: output slots [base, base + 32) of `order`, operand blocks
-// staged through X and B (32 x kStageStride double2 each, this warp's own shared memory).
+// staged through W (this warp's own shared memory).
 template <int TYPE, bool EXACT>
-__device__ __forceinline__ void warp_nd4_staged(const MultArgs& M, const int* __restrict__ order, int base, double2* X,
-                                                double2* B) {
-  constexpr int kStride = kStageStride;
+__device__ __forceinline__ void warp_nd4_staged(const MultArgs& M, const int* __restrict__ order, int base, unsigned char* W) {
   const unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int slot = base + lane;
   const bool has = slot < M.n_out;
   const int q = has ? order[slot] : 0;
-  int64_t t = has ? M.ptr[q] : 0, tend = has ? M.ptr[q + 1] : 0;
+  const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
+  const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
+  const int steps = __reduce_max_sync(kFull, nt);
   double acc[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = 0.0;
   const double2* Xg = reinterpret_cast<const double2*>(M.x);
   const double2* Bg = reinterpret_cast<const double2*>(M.b);
   const int chunk = lane & 7;
-  int2 pr_next = t < tend ? __ldcs(M.pairs + t) : make_int2(-1, -1);   // pair of the next step, loaded a step ahead
-  while (__any_sync(kFull, t < tend)) {
-    const bool act = t < tend;
-    const int2 pr = pr_next;
-    pr_next = t + 1 < tend ? __ldcs(M.pairs + t + 1) : make_int2(-1, -1);
+  const uint32_t w0 = smem_addr(W);
+  int2 pn = nt > 0 ? __ldcs(pairs) : make_int2(-1, -1);   // pair of the next step, loaded a step ahead
+  for (int t = 0; t < steps; ++t) {
+    const int2 pr = pn;
+    pn = t + 1 < nt ? __ldcs(pairs + t + 1) : make_int2(-1, -1);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int src = 4 * j + (lane >> 3);
       const int xb = __shfl_sync(kFull, pr.x, src);
       const int bb = __shfl_sync(kFull, pr.y, src);
+      const uint32_t d = w0 + src * 128 + ((chunk ^ (src & 7)) << 4);
       if (xb >= 0) {
-        X[src * kStride + chunk] = __ldg(Xg + (int64_t)xb * 8 + chunk);
-        B[src * kStride + chunk] = __ldg(Bg + (int64_t)bb * 8 + chunk);
+        cp_async16(d, Xg + (int64_t)xb * 8 + chunk);
+        cp_async16(d + 4096, Bg + (int64_t)bb * 8 + chunk);
       }
     }
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncwarp();
-    if (act) {
+    if (t < nt) {
       double x[16], b[16];
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const double2 xv = X[lane * kStride + v], bv = B[lane * kStride + v];
-        x[2 * v] = xv.x; x[2 * v + 1] = xv.y;
-        b[2 * v] = bv.x; b[2 * v + 1] = bv.y;
-      }
-      if (TYPE == 1) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-#pragma unroll
-          for (int n1 = 0; n1 < 4; ++n1) {
-            double a = acc[n1 + 4 * m];
-#pragma unroll
-            for (int n3 = 0; n3 < 4; ++n3) a = madd<EXACT>(a, x[n1 + 4 * n3], b[n3 + 4 * m]);
-            acc[n1 + 4 * m] = a;
-          }
-      } else {
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-#pragma unroll
-          for (int n1 = 0; n1 < 4; ++n1) {
-            double a = acc[n1 + 4 * m];
-#pragma unroll
-            for (int n2 = 0; n2 < 4; ++n2) a = madd<EXACT>(a, x[n1 + 4 * n2], b[m + 4 * n2]);
-            acc[n1 + 4 * m] = a;
-          }
-      }
-      ++t;
+      nd4_read(x, W, lane);
+      nd4_read(b, W + 4096, lane);
+      nd4_mul_add<TYPE, EXACT>(acc, x, b);
     }
     __syncwarp();
   }
@@ -344,12 +361,96 @@ __device__ __forceinline__ void warp_nd4_staged(const MultArgs& M, const int* __
 
 template <int TYPE, bool EXACT>
 __global__ void __launch_bounds__(128, 5) k_mult_nd4_warp(MultArgs M, const int* __restrict__ order) {
-  __shared__ double2 sx[4][32 * kStageStride];
-  __shared__ double2 sb[4][32 * kStageStride];
+  __shared__ __align__(128) unsigned char smem[4][kStageBytes];
   const int warp = threadIdx.x >> 5;
   const int base = (blockIdx.x * 4 + warp) * 32;
   if (base >= M.n_out) return;                  // whole warp
-  warp_nd4_staged<TYPE, EXACT>(M, order, base, sx[warp], sb[warp]);
+  warp_nd4_staged<TYPE, EXACT>(M, order, base, smem[warp]);
+}
+
+// Type 2, uniform 4 x 4 blocks: a(i, k) = sum over j in row k of B of c(i, j) b(k, j)^T.  All output blocks whose
+// column atom is an image of one atom kh read the same row of B in the same order, so a warp takes 32 of them
+// (one per lane) and walks that row: its B block is staged once per step and read by all lanes as a broadcast.
+// That halves the bytes from L2 per pair and the shared-memory reads of B.  Two stages: these products have few
+// output blocks, so an SM holds few warps.  Measured (512-atom cell, into the H range, 24064 output blocks): 0.325 ms
+// against 0.473 for the warp-staged and 0.546 for the four-lanes-per-block kernel; into the L range (63664) 0.600
+// against 0.601; three and four stages 0.766 and 0.878 there (the pair lists lose the L1).
+// tile: (kh's row start in B, its end, first entry of trans_dest for the outputs, their number).
+template <bool EXACT, int STAGES>
+__global__ void __launch_bounds__(64) k_mult_nd4_row(MultArgs M, const int4* __restrict__ tiles, int n_tiles,
+                                                     const int* __restrict__ trans_dest) {
+  constexpr int kBytes = 4096 + 128;              // one step: 32 X blocks and the B block
+  extern __shared__ __align__(128) unsigned char nd4_smem[];
+  const unsigned kFull = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = blockIdx.x * 2 + warp;
+  if (w >= n_tiles) return;                       // whole warp
+  unsigned char* W = nd4_smem + warp * STAGES * kBytes;
+  const int4 d = tiles[w];
+  const bool has = lane < d.w;
+  const int q = has ? trans_dest[d.z + lane] : 0;
+  double acc[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+  const double2* Xg = reinterpret_cast<const double2*>(M.x);
+  const double2* Bg = reinterpret_cast<const double2*>(M.b);
+  const int chunk = lane & 7;
+  const uint32_t w0 = smem_addr(W);
+  const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
+  const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
+  int taken = 0;
+  int2 pn = nt > 0 ? __ldg(pairs) : make_int2(-1, -1);      // the lane's next pair (its y is the B block)
+  int2 pn2 = nt > 1 ? __ldg(pairs + 1) : make_int2(-1, -1);
+  int eb = d.x;                                   // B block of the next step to stage
+  unsigned act = 0;                               // bit s: the lane has a term in the step staged s steps ago
+  auto issue = [&](int st) {
+    const bool mine = pn.y == eb;                 // eb >= 0: never true past the list's end
+    const int xl = mine ? pn.x : -1;
+    act = act << 1 | (mine ? 1u : 0u);
+    if (mine) {
+      ++taken;
+      pn = pn2;
+      pn2 = taken + 1 < nt ? __ldg(pairs + taken + 1) : make_int2(-1, -1);
+    }
+    if (eb < d.y) {
+      const uint32_t s = w0 + st * kBytes;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int src = 4 * j + (lane >> 3);
+        const int xb = __shfl_sync(kFull, xl, src);
+        if (xb >= 0) cp_async16(s + src * 128 + ((chunk ^ (src & 7)) << 4), Xg + (int64_t)xb * 8 + chunk);
+      }
+      if (lane < 8) cp_async16(s + 4096 + (lane << 4), Bg + (int64_t)eb * 8 + lane);
+    }
+    ++eb;
+    cp_async_commit();
+  };
+  int st = 0;
+#pragma unroll
+  for (int k = 0; k + 1 < STAGES; ++k) issue(k);
+  for (int e = d.x; e < d.y; ++e) {
+    issue(st + STAGES - 1 >= STAGES ? st - 1 : st + STAGES - 1);
+    cp_async_wait<STAGES - 1>();
+    __syncwarp();
+    if (act >> (STAGES - 1) & 1) {
+      const unsigned char* s = W + st * kBytes;
+      double x[16], b[16];
+      nd4_read(x, s, lane);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double2 v = *reinterpret_cast<const double2*>(s + 4096 + (k << 4));
+        b[2 * k] = v.x; b[2 * k + 1] = v.y;
+      }
+      nd4_mul_add<2, EXACT>(acc, x, b);
+    }
+    __syncwarp();
+    st = st + 1 == STAGES ? 0 : st + 1;
+  }
+  if (has) {
+    double2* O2 = reinterpret_cast<double2*>(M.out + 16 * (int64_t)q);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) __stcs(O2 + v, make_double2(acc[2 * v], acc[2 * v + 1]));
+  }
 }
 
 // Uniform 4 x 4 blocks, one thread per output block, operand blocks staged by the bulk-copy (TMA)
@@ -364,8 +465,6 @@ __global__ void __launch_bounds__(128, 5) k_mult_nd4_warp(MultArgs M, const int*
 // 2.59 ms on LS.L -> LSL is one copy per about 11 SM cycles, so the copy engine, not L1, bounds it.
 constexpr int kBulkStages = 3;
 constexpr int kBulkSlot = 144;            // bytes per staged block (128 + 16: conflict-free 16-byte reads)
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ bool warp_bar_wait(unsigned long long* bar, uint32_t parity, int* err) {
   const uint32_t a = smem_addr(bar);
@@ -489,16 +588,17 @@ __global__ void __launch_bounds__(128, 2) k_mult_nd4_bulk(MultArgs M, const int*
 }
 
 // Uniform 4 x 4 blocks, four lanes per output block: lane m of a quad owns column m of the block
-// (elements n1 + 4m, n1 = 0..3).  At each step the quad takes the next pair of its list: its lanes
-// load the first-operand block with two coalesced 16-byte loads each into shared memory, all four
-// read the whole block back (broadcast), and each lane loads the four B values of its column
-// straight into registers.  Four times the lanes of k_mult_nd4_warp, for products with few output
-// blocks and long pair lists (type 2 into the H and L ranges).  Every element keeps the order of
-// its terms, so the results are the same bits.
-template <int TYPE, bool EXACT>
-__global__ void __launch_bounds__(128, 8) k_mult_nd4_quad(MultArgs M, const int* __restrict__ order) {
-  constexpr int kStride = 9;                     // double2 per staged block (8 + 1 padding)
-  __shared__ double2 sx[4][8 * kStride];
+// (elements n1 + 4m, n1 = 0..3).  The quad copies the two blocks of a pair into its slots of a ring of
+// STAGES stages (cp.async, two 16-byte chunks of each block per lane), all four lanes read the X block as a
+// broadcast and each lane its column of B.  Four times the lanes of k_mult_nd4_warp, and STAGES - 1 pairs in
+// flight per quad, for products with few output blocks, whose time is the latency of their lists' steps.
+// Measured with 3, 4 and 6 stages: 64 atoms into the L range (1862 output blocks, 167 pairs each) 37.0, 35.0 and
+// 33.4 us (91 for the warp-staged kernel, 105 for one lane per element), 216 atoms L.S -> LS (115274) 23.0, 24.8
+// and 26.8 us (31.0 warp-staged).  Without the ring the 512-atom product into the H range took 0.545 ms; now 0.389.
+// Every element keeps the order of its terms, so the results are the same bits.
+template <int TYPE, bool EXACT, int STAGES>
+__global__ void __launch_bounds__(128) k_mult_nd4_quad(MultArgs M, const int* __restrict__ order) {
+  __shared__ __align__(128) unsigned char smem[4][STAGES][8 * 256];   // per quad: the X block, then the B block
   const unsigned kFull = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int qd = lane >> 2, m = lane & 3;
@@ -507,39 +607,55 @@ __global__ void __launch_bounds__(128, 8) k_mult_nd4_quad(MultArgs M, const int*
   const int slot = base + qd;
   const bool has = slot < M.n_out;
   const int q = has ? order[slot] : 0;
-  int64_t t = has ? M.ptr[q] : 0;
-  const int64_t tend = has ? M.ptr[q + 1] : 0;
+  const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
+  const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
+  const int steps = __reduce_max_sync(kFull, nt);
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  double2* X = sx[warp] + qd * kStride;          // this quad's staged block
   const double2* Xg = reinterpret_cast<const double2*>(M.x);
   const double2* Bg = reinterpret_cast<const double2*>(M.b);
-  int2 pr_next = t < tend ? __ldcs(M.pairs + t) : make_int2(-1, -1);   // pair of the next step, loaded a step ahead
-  while (__any_sync(kFull, t < tend)) {
-    const bool act = t < tend;                   // uniform over the quad
-    const int2 pr = pr_next;
-    pr_next = t + 1 < tend ? __ldcs(M.pairs + t + 1) : make_int2(-1, -1);
-    double bc[4];
-    if (act) {
-      X[m] = __ldg(Xg + (int64_t)pr.x * 8 + m);
-      X[m + 4] = __ldg(Xg + (int64_t)pr.x * 8 + m + 4);
-      if (TYPE == 1) {
-        // B[n3 + 4m], n3 = 0..3: the four contiguous values of column m
-        const double2 u = __ldg(Bg + (int64_t)pr.y * 8 + 2 * m), v = __ldg(Bg + (int64_t)pr.y * 8 + 2 * m + 1);
-        bc[0] = u.x; bc[1] = u.y; bc[2] = v.x; bc[3] = v.y;
-      } else {
-        // B[m + 4 n2], n2 = 0..3: for each n2 the quad reads one 32-byte sector
-        const double* Bb = M.b + (int64_t)pr.y * 16 + m;
-#pragma unroll
-        for (int n2 = 0; n2 < 4; ++n2) bc[n2] = __ldg(Bb + 4 * n2);
-      }
+  // chunk v of a block lies at chunk v ^ qd: the eight quads' reads of one chunk fall into different banks
+  const int c0 = (m ^ qd) << 4, c1 = ((m + 4) ^ qd) << 4;
+  int issued = 0;
+  int2 pn = nt > 0 ? __ldcs(pairs) : make_int2(0, 0);    // the next pair to copy, loaded a step ahead
+  auto issue = [&](int st) {
+    if (issued < nt) {
+      const uint32_t d = smem_addr(smem[warp][st]) + qd * 256;
+      const double2 *xs = Xg + (int64_t)pn.x * 8 + m, *bs = Bg + (int64_t)pn.y * 8 + m;
+      cp_async16(d + c0, xs);
+      cp_async16(d + c1, xs + 4);
+      cp_async16(d + 128 + c0, bs);
+      cp_async16(d + 128 + c1, bs + 4);
+      if (issued + 1 < nt) pn = __ldcs(pairs + issued + 1);
     }
+    ++issued;
+    cp_async_commit();
+  };
+  int st = 0;
+#pragma unroll
+  for (int k = 0; k + 1 < STAGES; ++k) issue(k);
+  for (int t = 0; t < steps; ++t) {
+    issue(st == 0 ? STAGES - 1 : st - 1);
+    cp_async_wait<STAGES - 1>();
     __syncwarp();
-    if (act) {
-      double x[16];
+    if (t < nt) {
+      const unsigned char* X = smem[warp][st] + qd * 256;
+      const unsigned char* B = X + 128;
+      double x[16], bc[4];
 #pragma unroll
       for (int v = 0; v < 8; ++v) {
-        const double2 xv = X[v];
+        const double2 xv = *reinterpret_cast<const double2*>(X + ((v ^ qd) << 4));
         x[2 * v] = xv.x; x[2 * v + 1] = xv.y;
+      }
+      if (TYPE == 1) {
+        // B[n3 + 4m], n3 = 0..3: the four contiguous values of column m
+        const double2 u = *reinterpret_cast<const double2*>(B + (((2 * m) ^ qd) << 4));
+        const double2 v = *reinterpret_cast<const double2*>(B + (((2 * m + 1) ^ qd) << 4));
+        bc[0] = u.x; bc[1] = u.y; bc[2] = v.x; bc[3] = v.y;
+      } else {
+        // B[m + 4 n2], n2 = 0..3
+#pragma unroll
+        for (int n2 = 0; n2 < 4; ++n2)
+          bc[n2] = *reinterpret_cast<const double*>(B + (((2 * n2 + (m >> 1)) ^ qd) << 4) + ((m & 1) << 3));
       }
       // type 1: acc[n1] += sum_n3 x[n1 + 4 n3] B[n3 + 4m]; type 2: acc[n1] += sum_n2 x[n1 + 4 n2] B[m + 4 n2]
 #pragma unroll
@@ -549,9 +665,9 @@ __global__ void __launch_bounds__(128, 8) k_mult_nd4_quad(MultArgs M, const int*
         for (int n = 0; n < 4; ++n) a = madd<EXACT>(a, x[n1 + 4 * n], bc[n]);
         acc[n1] = a;
       }
-      ++t;
     }
-    __syncwarp();
+    __syncwarp();                                // the stage is read before the next issue() refills it
+    st = st + 1 == STAGES ? 0 : st + 1;
   }
   if (has) {
     double2* O2 = reinterpret_cast<double2*>(M.out + 16 * (int64_t)q) + 2 * m;
@@ -678,17 +794,6 @@ struct GroupShape {
   static constexpr int kStage = kBlocks * (kStrideX + kStrideB);      // the X blocks, then the B blocks
   static constexpr int kWarpBytes = STAGES * kStage;
 };
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 
 // n doubles at src (8-byte aligned) to the 16-byte aligned slot dst, by the LPB lanes l of a group; the data
 // starts at dst + 8 when src is not 16-byte aligned.  Reads no byte outside [src, src + n).
@@ -896,15 +1001,14 @@ struct BatchParams {
 };
 static_assert(sizeof(BatchParams) < 32000, "batched product table exceeds the kernel parameter space");
 
-constexpr int kBatchWarpBytes = 2 * 32 * kStageStride * 16;    // the warp-staged 4 x 4 kernel's X and B
+constexpr int kBatchWarpBytes = kStageBytes + 256;    // the larger of the two kernels' staging areas
 static_assert(GroupShape<13, 16, 1>::kWarpBytes <= kBatchWarpBytes && GroupShape<16, 16, 1>::kWarpBytes <= kBatchWarpBytes,
               "batched warps share one staging area");
 
 template <int TYPE, bool EXACT>
 __device__ __forceinline__ void batch_unit(const BatchProduct& P, int family, int unit, unsigned char* W) {
   if (family == kBatchNd4) {
-    double2* X = reinterpret_cast<double2*>(W);
-    warp_nd4_staged<TYPE, EXACT>(P.M, P.order, unit * 32, X, X + 32 * kStageStride);
+    warp_nd4_staged<TYPE, EXACT>(P.M, P.order, unit * 32, W);
   } else if (family == kBatchU13) {
     warp_group<TYPE, EXACT, 13, 13, 16, 1>(P.M, P.order, unit * 2, W);
   } else if (family == kBatchMax13) {
@@ -1068,7 +1172,7 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   const int T = 256;
   RangeIndex& O = P.mult_type == 1 ? *S.ranges[P.rc] : *S.ranges[P.ra];
   RangeIndex& X = P.mult_type == 1 ? *S.ranges[P.ra] : *S.ranges[P.rc];
-  if (nd4 && (variant == 3 || variant == 5 || variant == 6)) ensure_order(S, P);
+  if (nd4 && (variant >= 3)) ensure_order(S, P);
   if (nd4 && variant == 6) {
     const int grid = (M.n_out + 127) / 128;
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
@@ -1085,13 +1189,28 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   } else if (nd4 && variant == 5) {
     const int grid = (M.n_out + 31) / 32;        // 8 output blocks per warp, 4 warps per CTA
     if (P.mult_type == 1) {
-      if (exact) k_mult_nd4_quad<1, true><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_quad<1, false><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_quad<1, true, 4><<<grid, 128, 0, st>>>(M, P.order.p);
+      else k_mult_nd4_quad<1, false, 4><<<grid, 128, 0, st>>>(M, P.order.p);
     } else {
-      if (exact) k_mult_nd4_quad<2, true><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_quad<2, false><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_quad<2, true, 4><<<grid, 128, 0, st>>>(M, P.order.p);
+      else k_mult_nd4_quad<2, false, 4><<<grid, 128, 0, st>>>(M, P.order.p);
     }
-  } else if (nd4 && variant == 3) {
+  } else if (nd4 && variant == 4 && P.mult_type == 2) {
+    if (P.n_row_tiles < 0) {
+      // up to 32 output blocks whose column atoms are images of one atom, with that atom's row of B
+      RangeIndex& B = *S.ranges[P.rb];
+      std::vector<int4> tl;
+      for (int k = 0; k < S.geo.n_prim; ++k)
+        for (int z = O.h_row_ptr[k]; z < O.h_row_ptr[k + 1]; z += 32)
+          tl.push_back(make_int4(B.h_row_ptr[k], B.h_row_ptr[k + 1], z, std::min(32, O.h_row_ptr[k + 1] - z)));
+      P.row_tiles.upload(tl, st);
+      P.n_row_tiles = (int)tl.size();
+    }
+    constexpr int kSt = 2;
+    const int smem = 2 * kSt * (4096 + 128), grid = (P.n_row_tiles + 1) / 2;
+    if (exact) k_mult_nd4_row<true, kSt><<<grid, 64, smem, st>>>(M, P.row_tiles.p, P.n_row_tiles, O.trans_dest.p);
+    else k_mult_nd4_row<false, kSt><<<grid, 64, smem, st>>>(M, P.row_tiles.p, P.n_row_tiles, O.trans_dest.p);
+  } else if (nd4 && (variant == 3 || variant == 4)) {
     const int grid = (M.n_out + 127) / 128;
     if (P.mult_type == 1) {
       if (exact) k_mult_nd4_warp<1, true><<<grid, 128, 0, st>>>(M, P.order.p);
@@ -1170,48 +1289,33 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   CQ_CUDA(cudaGetLastError());
 }
 
-// Autotuner: on the first call of a product, time the candidate kernels (one warm launch each,
-// then three rounds in which every candidate runs once between CUDA events on the system's
-// stream; a candidate's time is its fastest round) and keep the fastest for the plan; a later
-// candidate replaces the preferred one only when it is at least 5 % faster.  The candidates give identical
-// bits and each fully overwrites the output, so tuning changes speed only; the last timed launch
-// leaves the correct result.
-static int tuned_variant(System& S, ProductPlan& P, const MultArgs& M, int exact, bool nd4) {
-  if (!nd4) {                      // untimed: the generic kernel is 3 to 5 times slower on every product
+// Kernel of an FP64 product when none is forced: a rule on the product's sizes (every kernel gives the same bits).
+// Timing the candidates on a product's first call, as this library once did, cost a new geometry several times
+// the product and chose wrongly while other streams kept the device busy.  Measured on cells of 64 to 1000 atoms
+// and ranges of 8 to 26 bohr (warp-staged / four lanes per block / row kernel, us):
+//  - type 1: four lanes per block below 180,000 output blocks (7940: 12.9 / 7.9; 85,546: 37.5 / 22.9; 163,036: 27.1 /
+//    27.0; 217,306: 31.2 / 33.2; 1,182,142: 580 / 716);
+//  - type 2: four lanes per block below 20,000 output blocks (7940 with 532 pairs each: 302 / 148 / 234; 18,048: 465 /
+//    248 / 316; 24,064: 472 / 378 / 322); above, the row kernel, whose steps are the rows of B: where the lists
+//    hold most of those rows, and from 40,000 blocks on (every SM full) also most lanes have a block (63,664 with
+//    97 % of the lanes: 605 / 823 / 570; 47,000 with 73 %: 520 / 625 / 611; lists of 88 %: 127 / 170 / 135).
+// Other block sizes and unaligned operands: the group kernel (the generic one is 3 to 5 times slower).
+static int auto_variant(System& S, ProductPlan& P, int n_out, bool nd4) {
+  if (!nd4) {
     if (S.uniform_nsf != 4) P.tuned = 4;
     return 4;
   }
   if (P.tuned >= 0) return P.tuned;
-  // candidates of uniform 4x4 blocks, the preferred kernel first: warp-staged, four lanes per
-  // block, thread per block, 16 lanes per block (the last two the most parallel, for products with
-  // few output blocks)
-  // (variant 6, the bulk-copy-staged kernel, is not a candidate: 2.4x slower than variant 3 on every
-  // product of the 512-atom SZ chain, since one 128-byte bulk copy takes about 11 SM cycles)
-  const int cands[4] = {3, 5, 1, 0};
-  const int nc = 4;
-  cudaEvent_t e0, e1;
-  CQ_CUDA(cudaEventCreate(&e0));
-  CQ_CUDA(cudaEventCreate(&e1));
-  float best[4] = {1e30f, 1e30f, 1e30f, 1e30f};
-  for (int c = 0; c < nc; ++c) launch_variant(S, P, M, cands[c], exact, nd4);
-  for (int round = 0; round < 3; ++round)
-    for (int c = 0; c < nc; ++c) {
-      CQ_CUDA(cudaEventRecord(e0, S.stream));
-      launch_variant(S, P, M, cands[c], exact, nd4);
-      CQ_CUDA(cudaEventRecord(e1, S.stream));
-      CQ_CUDA(cudaEventSynchronize(e1));
-      float ms = 0.f;
-      CQ_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      best[c] = std::min(best[c], ms);
-    }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  int pick = 0;
-  for (int c = 1; c < nc; ++c)
-    if (best[c] < 0.95f * best[pick]) pick = c;
-  for (int c = 0; c < nc; ++c) P.tune_ms[cands[c]] = best[c];
-  P.tuned = cands[pick];
-  return P.tuned;
+  if (P.mult_type == 1) return P.tuned = n_out < 180000 ? 5 : 3;
+  if (n_out < 20000) return P.tuned = 5;
+  const std::vector<int>&o = S.ranges[P.ra]->h_row_ptr, &b = S.ranges[P.rb]->h_row_ptr;
+  int64_t steps = 0, tiles = 0;                  // pairs if every list held its whole row of B; groups of 32 blocks
+  for (int k = 0; k < S.geo.n_prim; ++k) {
+    steps += (int64_t)(o[k + 1] - o[k]) * (b[k + 1] - b[k]);
+    tiles += (o[k + 1] - o[k] + 31) / 32;
+  }
+  const double lists = (double)P.n_pairs / (double)std::max<int64_t>(steps, 1), lanes = n_out / (32.0 * (double)tiles);
+  return P.tuned = n_out < 40000 ? (lists >= 0.75 ? 4 : 3) : (lists >= 0.9 && lanes >= 0.8 ? 4 : 3);
 }
 
 // kernel arguments of one product (roles of mat_mult: type 1 writes c from a, b; type 2 writes a from c, b);
@@ -1258,7 +1362,7 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
     CQ_CUDA(cudaGetLastError());
   } else {
     int variant = S.mult_variant;
-    if (variant == kVariantAuto) variant = tuned_variant(S, P, M, exact, nd4);
+    if (variant == kVariantAuto) variant = auto_variant(S, P, M.n_out, nd4);
     launch_variant(S, P, M, variant, exact, nd4);
   }
   if (S.prof.on) {

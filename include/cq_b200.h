@@ -182,9 +182,9 @@ int cq_grab_matrix(cq_system* sys, int r, double* a_dev, const char* path, int64
 /* Algorithmic work of one product: (k,i,j) triples with a stored result and 2*sum nd^3 flops. */
 int cq_product_work(cq_system* sys, int mult_type, int ra, int rb, int rc, int64_t* triples, int64_t* flops);
 
-/* Autotuner record of one product: the FP64 kernel variant it chose (-1 before the product's
- * first autotuned call) and the timed milliseconds of each candidate variant (ms[7], 0 = not
- * timed); for its split-precision form the output blocks per warp it chose (1, 2, 4 or 8; -1 =
+/* Kernel record of one product: the FP64 kernel variant chosen for it (-1 before the product's
+ * first call with the automatic choice) and the timed milliseconds of each variant (ms[7], 0 = not
+ * timed; the FP64 choice is a rule and times none); for its split-precision form the output blocks per warp it chose (1, 2, 4 or 8; -1 =
  * not tuned yet) and the timed milliseconds of those four group sizes (group_ms[4]). */
 int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int* variant, float* ms, int* group,
                       float* group_ms);
@@ -268,17 +268,17 @@ int cq_launch_count(cq_system* sys, int64_t* count);
  * hamiltonian_H up to the last bit of exp(). */
 int cq_generate_SH(cq_system* sys, int r, int which, uint64_t seed, double* out);
 
-/* Tuning options.  CQ_OPT_MULT_VARIANT: FP64 4x4 product kernel, -1 = chosen per product by the
- * autotuner (default: the first call of each product times the candidate kernels with CUDA
- * events and keeps the fastest), 0 = one lane per output element, 1 = one thread per output
+/* Tuning options.  CQ_OPT_MULT_VARIANT: FP64 4x4 product kernel, -1 = chosen per product by a rule on
+ * its sizes (default), 0 = one lane per output element, 1 = one thread per output
  * block, 2 = one thread per output block with the first operand's row staged in shared memory,
  * 3 = one thread per output block with the warp staging the operand blocks through shared
  * memory, 5 = four lanes per output block (one column each), the first operand's block staged
- * in shared memory, 6 = one thread per output block with its operand blocks staged by bulk copies
+ * in shared memory, 4 = mult type 2: as 3 with the row of B that the blocks of a warp share staged once
+ * (type 1: as 3), 6 = one thread per output block with its operand blocks staged by bulk copies
  * (cp.async.bulk, completion on an mbarrier, bounded waits); for other block sizes (DZP 13 x 13,
  * mixed sizes) 0 = one warp per output block, one lane per element, 4 = two or four output blocks per
- * warp, their operand blocks staged in shared memory, whole columns per lane (the autotuner candidates are
- * 3/5/1/0 for uniform 4 x 4 blocks, and 4 is used untimed otherwise; variant 6 is selectable only).  All give
+ * warp, their operand blocks staged in shared memory, whole columns per lane (-1 chooses among
+ * 3 and 5, and 4 for mult type 2, for uniform 4 x 4 blocks, and 4 otherwise; the others are selectable only).  All give
  * identical results.
  * CQ_OPT_BLOCKING_SYNC: 1 = the host thread sleeps on a blocking-sync event whenever the
  * solver waits for a scalar from the device (many concurrent solvers per host core), 0 = it

@@ -51,3 +51,31 @@ def test_group_kernel_bits(sizes, mult_type):
         cq_b200.mat_mult_batch([(g, mult_type, 0, 1, 2, *dev, cq_b200.PREC_FP64)])
         g.synchronize()
         assert np.array_equal(dev[out].cpu().numpy(), ref[out])
+
+
+@pytest.mark.parametrize("shape", ["cell", "cluster33", "cluster1"])
+@pytest.mark.parametrize("exact", [True, False])
+def test_4x4_kernels_give_the_same_bits(shape, exact):
+    """The staged 4 x 4 kernels against the unstaged one (one lane per element, checked against the oracle elsewhere):
+    full and ragged groups of output blocks, pair lists that hold a whole row of B and lists that hold part of it
+    (the input range shorter than the sum of the others), both mult types."""
+    import torch
+    import cq_b200
+    coords, cell = {"cell": lambda: inputs.diamond_si(2, sigma=0.1, seed=51),
+                    "cluster33": lambda: inputs.si_cluster(33, sigma=0.1, seed=52),
+                    "cluster1": lambda: inputs.si_cluster(1, sigma=0.0, seed=53)}[shape]()
+    g = cq_b200.System(coords, cell, np.full(len(coords), 4, np.int32), [10.0, 8.0, 18.0, 14.0])
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    for t, rc in ((1, 2), (1, 3), (2, 2), (2, 3)):
+        ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for r in (0, 1, rc)]
+        out = 2 if t == 1 else 0
+        ref = None
+        for v in (0, 3, 4, 5, -1):
+            g.set_mult_variant(v)
+            ops[out].fill_(float("nan"))
+            torch.cuda.synchronize()
+            g.mat_mult(t, 0, 1, rc, *ops, exact=exact)
+            g.synchronize()
+            ref = ops[out].clone() if ref is None else ref
+            assert torch.equal(ops[out], ref), (t, rc, v)
