@@ -19,7 +19,7 @@ namespace cqb {
 namespace {
 
 constexpr int kT = 256;
-constexpr int kRedBlocks = 1184;   // 148 SMs x 8: the largest grid of the exact sums
+constexpr int kRedBlocks = 592;    // 148 SMs x 4: the largest grid of one exact sum
 
 int grid_for(int64_t n) {
   int64_t b = (n + kT - 1) / kT;
@@ -69,18 +69,55 @@ __global__ void k_masked_add(int nnz, const int* __restrict__ partner, const int
   const double* B = b + b_elem[pb];
   for (int t = lane; t < ne; t += 32) A[t] = __dadd_rn(__dmul_rn(alpha, A[t]), __dmul_rn(beta, B[t]));
 }
-// AT(dest) = A(e)^T
-__global__ void k_transpose(int nnz, const int* __restrict__ dest, const int64_t* __restrict__ elem,
-                            const int* __restrict__ row, const int* __restrict__ cover, const int* __restrict__ prim_nsf,
-                            const int* __restrict__ cover_nsf, const double* __restrict__ a, double* __restrict__ at) {
+// the same for uniform 4 x 4 blocks with 16-byte aligned arrays: eight lanes per block, one double2 each (a warp per
+// block would leave half of its lanes idle and look up four index arrays per block)
+__global__ void __launch_bounds__(kT) k_masked_add_nd4(int nnz, const int* __restrict__ partner, double2* __restrict__ a,
+                                                       double alpha, const double2* __restrict__ b, double beta) {
+  const int64_t stride = (int64_t)gridDim.x * kT;
+  for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < (int64_t)nnz * 8; i += stride) {
+    const int pb = partner[i >> 3];
+    if (pb < 0) continue;
+    double2 x = a[i];
+    const double2 y = b[(int64_t)pb * 8 + (i & 7)];
+    x.x = __dadd_rn(__dmul_rn(alpha, x.x), __dmul_rn(beta, y.x));
+    x.y = __dadd_rn(__dmul_rn(alpha, x.y), __dmul_rn(beta, y.y));
+    a[i] = x;
+  }
+}
+// AT(dest) = A(e)^T: a warp per block, through shared memory so that both the read and the write run along memory
+__global__ void __launch_bounds__(kT) k_transpose(int nnz, const int* __restrict__ dest, const int64_t* __restrict__ elem,
+                                                  const int* __restrict__ row, const int* __restrict__ cover,
+                                                  const int* __restrict__ prim_nsf, const int* __restrict__ cover_nsf,
+                                                  const double* __restrict__ a, double* __restrict__ at) {
+  __shared__ double tile[kT / 32][256];
   int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e >= nnz) return;
   int ndi = prim_nsf[row[e]], ndj = cover_nsf[cover[e]];
   const double* A = a + elem[e];
   double* T = at + elem[dest[e]];
-  for (int t = lane; t < ndi * ndj; t += 32) {
-    int n1 = t % ndi, n2 = t / ndi;
-    T[n2 + ndj * n1] = A[t];
+  double* W = tile[threadIdx.x >> 5];
+  const int ne = ndi * ndj, magic = 65536 / ndj + 1;      // t / ndj = t * magic >> 16 for t < 256, ndj <= 16
+  for (int t = lane; t < ne; t += 32) W[t] = A[t];
+  __syncwarp();
+  for (int t = lane; t < ne; t += 32) {                   // element (n2, n1) of the transpose
+    const int n1 = (t * magic) >> 16, n2 = t - n1 * ndj;
+    T[t] = W[n1 + ndi * n2];
+  }
+}
+// the same for uniform 4 x 4 blocks with 16-byte aligned arrays: eight lanes per block; lane (n1 pair, n2) reads two
+// values of column n2 and trades one with the lane of column n2 ^ 1, so that it writes two neighbours as well.
+// Memory bound: 151 MB read and written (42-bohr range of 512 atoms) in 54.9 us against 236.9 us with a warp per block.
+__global__ void __launch_bounds__(kT) k_transpose_nd4(int nnz, const int* __restrict__ dest, const double2* __restrict__ a,
+                                                      double2* __restrict__ at) {
+  const int64_t stride = (int64_t)gridDim.x * kT, n = (int64_t)nnz * 8;
+  const int64_t n32 = (n + 31) & ~(int64_t)31;            // whole warps: the shuffle needs every lane
+  for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n32; i += stride) {
+    const double2 v = i < n ? a[i] : make_double2(0.0, 0.0);
+    const int r = (int)(i & 1), c = (int)(i >> 1) & 3;     // rows 2r, 2r + 1 of column c
+    const double got = __shfl_xor_sync(0xffffffffu, c & 1 ? v.x : v.y, 2);
+    // even column: row 2r of columns c, c + 1; odd column: row 2r + 1 of columns c - 1, c
+    const double2 w = c & 1 ? make_double2(got, v.y) : make_double2(v.x, got);
+    if (i < n) at[(int64_t)dest[i >> 3] * 8 + 2 * (2 * r + (c & 1)) + (c >> 1)] = w;
   }
 }
 // ---------------------------------------------------------------------------
@@ -109,22 +146,23 @@ __device__ __forceinline__ void acc_add(Acc192& a, const Acc192& b) {
 }
 // term v -> fixed point with lsb 2^lsb_exp (exact for every bit at or above the lsb)
 __device__ __forceinline__ void acc_term(Acc192& a, double v, int lsb_exp) {
-  if (v == 0.0) return;
-  int e;
-  double f = frexp(v, &e);                              // v = f 2^e, 0.5 <= |f| < 1
-  long long m = (long long)ldexp(f, 53);                // exact, |m| < 2^53
-  bool neg = m < 0;
-  uint64_t mag = (uint64_t)(neg ? -m : m);
-  int s = e - 53 - lsb_exp;                             // bit position of m's lsb
+  const uint64_t u = (uint64_t)__double_as_longlong(v);
+  const int ef = (int)(u >> 52) & 0x7ff;
+  uint64_t mag = u & 0xfffffffffffffull;                // v = mag 2^(max(ef, 1) - 1075)
+  if (ef) mag |= 1ull << 52;
+  if (mag == 0) return;
+  const int s = (ef ? ef : 1) - 1075 - lsb_exp;         // bit position of mag's lsb
   Acc192 t = {{0, 0, 0}};
   if (s >= 0) {
-    int idx = s >> 6, off = s & 63;
-    if (idx < 3) t.w[idx] = mag << off;
-    if (off && idx + 1 < 3) t.w[idx + 1] = mag >> (64 - off);
+    const int idx = s >> 6, off = s & 63;
+    const uint64_t lo = mag << off, hi = off ? mag >> (64 - off) : 0;
+    t.w[0] = idx == 0 ? lo : 0;
+    t.w[1] = idx == 1 ? lo : idx == 0 ? hi : 0;
+    t.w[2] = idx == 2 ? lo : idx == 1 ? hi : 0;
   } else if (-s < 64) {
     t.w[0] = mag >> (-s);
   }
-  if (neg) {                                            // two's complement negation
+  if (u >> 63) {                                        // two's complement negation
     t.w[0] = ~t.w[0]; t.w[1] = ~t.w[1]; t.w[2] = ~t.w[2];
     Acc192 one = {{1, 0, 0}};
     acc_add(t, one);
@@ -134,59 +172,99 @@ __device__ __forceinline__ void acc_term(Acc192& a, double v, int lsb_exp) {
 __device__ __forceinline__ double dterm(const double* x, const double* y, int64_t i) {
   return y ? __dmul_rn(x[i], y[i]) : x[i];
 }
-// pass 1: largest exponent of the nonzero terms, stored biased by kEBias (0 = every term is zero);
-// a non-finite term sets the flag.  Both words start at zero (cudaMemsetAsync).
-__global__ void k_acc_emax(const double* __restrict__ x, const double* __restrict__ y, int64_t n, int* __restrict__ emax,
-                           int* __restrict__ nonfinite) {
+// The sums of one call: operands, lengths and grid of each.
+struct SumArgs {
+  const double* x[kSumSlots];
+  const double* y[kSumSlots];
+  int64_t n[kSumSlots];
+  int blocks[kSumSlots];
+};
+// Scratch of a sum: flags (largest biased exponent, non-finite, blocks done), zero between calls (the last block of
+// pass 2 clears them), and the block partials.
+constexpr int kSumFlags = 3;
+
+// pass 1 of sum blockIdx.y: largest frexp exponent of the nonzero terms, stored biased by kEBias (0 = every term is
+// zero); a non-finite term sets the flag
+__global__ void __launch_bounds__(kT) k_acc_emax(const __grid_constant__ SumArgs A, int* __restrict__ flags) {
+  const int k = blockIdx.y;
+  if (blockIdx.x >= A.blocks[k]) return;
+  const double *x = A.x[k], *y = A.y[k];
+  const int64_t n = A.n[k], stride = (int64_t)A.blocks[k] * kT;
   int best = 0;
   bool bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n; i += (int64_t)gridDim.x * kT) {
-    double v = dterm(x, y, i);
-    if (!isfinite(v)) { bad = true; continue; }
-    if (v != 0.0) { int e; frexp(v, &e); best = max(best, e + kEBias); }
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n; i += stride) {
+    const uint64_t u = (uint64_t)__double_as_longlong(dterm(x, y, i));
+    const int ef = (int)(u >> 52) & 0x7ff;
+    const uint64_t frac = u & 0xfffffffffffffull;
+    if (ef == 0x7ff) bad = true;
+    else if (ef) best = max(best, ef - 1022 + kEBias);
+    else if (frac) best = max(best, 64 - __clzll((long long)frac) - 1074 + kEBias);
   }
-  for (int o = 16; o; o >>= 1) best = max(best, __shfl_down_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0 && best != 0) atomicMax(emax, best);
-  if (bad) atomicExch(nonfinite, 1);
+  best = __reduce_max_sync(0xffffffffu, best);
+  if ((threadIdx.x & 31) == 0 && best != 0) atomicMax(flags + kSumFlags * k, best);
+  if (bad) atomicExch(flags + kSumFlags * k + 1, 1);
 }
-__device__ void block_acc_reduce(Acc192 a, uint64_t* __restrict__ out) {
-  __shared__ uint64_t s[3][kT];
-  for (int k = 0; k < 3; ++k) s[k][threadIdx.x] = a.w[k];
+// sum over the block of every thread's a, valid in thread 0
+__device__ Acc192 block_acc_reduce(Acc192 a) {
+  __shared__ uint64_t s[3][kT / 32];
+  for (int o = 16; o; o >>= 1) {
+    Acc192 z;
+    for (int k = 0; k < 3; ++k) z.w[k] = __shfl_down_sync(0xffffffffu, a.w[k], o);
+    acc_add(a, z);
+  }
+  const int warp = threadIdx.x >> 5;
   __syncthreads();
-  for (int w = kT / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      Acc192 x = {{s[0][threadIdx.x], s[1][threadIdx.x], s[2][threadIdx.x]}};
-      Acc192 z = {{s[0][threadIdx.x + w], s[1][threadIdx.x + w], s[2][threadIdx.x + w]}};
-      acc_add(x, z);
-      for (int k = 0; k < 3; ++k) s[k][threadIdx.x] = x.w[k];
+  if ((threadIdx.x & 31) == 0) for (int k = 0; k < 3; ++k) s[k][warp] = a.w[k];
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kT / 32; ++w) {
+      const Acc192 z = {{s[0][w], s[1][w], s[2][w]}};
+      acc_add(a, z);
     }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) for (int k = 0; k < 3; ++k) out[k] = s[k][0];
+  return a;
 }
-// pass 2: fixed-point accumulation, one 192-bit partial per block (zero when pass 1 found no
-// nonzero term or a non-finite one: the host reports 0 or NaN from the flags)
-__global__ void __launch_bounds__(kT) k_acc_sum(const double* __restrict__ x, const double* __restrict__ y, int64_t n,
-                                                const int* __restrict__ flags, uint64_t* __restrict__ part) {
+// pass 2 of sum blockIdx.y: fixed-point accumulation, one 192-bit partial per block (zero when pass 1 found no
+// nonzero term or a non-finite one: the host reports 0 or NaN from the flags); the block that finishes last adds the
+// partials into out[4 k .. 4 k + 2], puts the flags into out[4 k + 3] and clears them.  What bounds the two passes for
+// the chain's matrices is launches and their gaps: all sums of a call share the two launches, and `out` is pinned
+// host memory, so no memset, final pass or copy follows them.
+__global__ void __launch_bounds__(kT) k_acc_sum(const __grid_constant__ SumArgs A, int* __restrict__ flags,
+                                                uint64_t* __restrict__ part, int part_stride, uint64_t* __restrict__ out) {
+  __shared__ int last;
+  const int k = blockIdx.y, nb = A.blocks[k];
+  if (blockIdx.x >= nb) return;
+  const double *x = A.x[k], *y = A.y[k];
+  const int64_t n = A.n[k], stride = (int64_t)nb * kT;
+  int* f = flags + kSumFlags * k;
+  uint64_t* p = part + (size_t)k * part_stride;
+  const int eb = f[0], bad = f[1];
   Acc192 a = {{0, 0, 0}};
-  const int eb = flags[0];
-  if (eb != 0 && flags[1] == 0) {
+  if (eb != 0 && bad == 0) {
     const int lsb = eb - kEBias - kAccFrac;
-    for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n; i += (int64_t)gridDim.x * kT)
-      acc_term(a, dterm(x, y, i), lsb);
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n; i += stride) acc_term(a, dterm(x, y, i), lsb);
   }
-  block_acc_reduce(a, part + 3 * blockIdx.x);
-}
-// pass 3: sum of the block partials into out[0..2]; out[3] carries the flags of pass 1
-__global__ void __launch_bounds__(kT) k_acc_final(const uint64_t* __restrict__ part, int nb, const int* __restrict__ flags,
-                                                  uint64_t* __restrict__ out) {
-  Acc192 a = {{0, 0, 0}};
+  a = block_acc_reduce(a);
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < 3; ++w) p[3 * blockIdx.x + w] = a.w[w];
+    __threadfence();
+    last = atomicAdd(f + 2, 1) == nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  Acc192 t = {{0, 0, 0}};
   for (int b = threadIdx.x; b < nb; b += kT) {
-    Acc192 t = {{part[3 * b], part[3 * b + 1], part[3 * b + 2]}};
-    acc_add(a, t);
+    const Acc192 z = {{__ldcg(p + 3 * b), __ldcg(p + 3 * b + 1), __ldcg(p + 3 * b + 2)}};
+    acc_add(t, z);
   }
-  block_acc_reduce(a, out);
-  if (threadIdx.x == 0) out[3] = (uint64_t)(uint32_t)flags[0] | ((uint64_t)(uint32_t)flags[1] << 32);
+  t = block_acc_reduce(t);
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < 3; ++w) out[4 * k + w] = t.w[w];
+    out[4 * k + 3] = (uint64_t)(uint32_t)eb | ((uint64_t)(uint32_t)bad << 32);
+    f[0] = f[1] = f[2] = 0;
+  }
 }
 // store_matrix_value(..., j, j, one) on every onsite block: the diagonal of each atom's self block
 __global__ void k_set_onsite_diag(int n_prim, const int64_t* __restrict__ onsite, const int* __restrict__ prim_nsf,
@@ -276,9 +354,13 @@ void dev_matrix_add(System& S, int ra, double* a, double alpha, int rb, const do
   RangeIndex &A = *S.ranges[ra], &B = *S.ranges[rb];
   AddMap& m = get_addmap(S, ra, rb);
   if (A.nnz == 0) return;
-  k_masked_add<<<(int)(((int64_t)A.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
-      A.nnz, m.partner.p, A.nb_elem.p, B.nb_elem.p, A.nb_row.p, A.nb_cover.p, S.dg.prim_nsf.p, S.dg.cover_nsf.p, a, alpha,
-      b, beta);
+  if (S.uniform_nsf == 4 && ((uintptr_t)a | (uintptr_t)b) % 16 == 0)
+    k_masked_add_nd4<<<grid_for((int64_t)A.nnz * 8), kT, 0, S.stream>>>(
+        A.nnz, m.partner.p, reinterpret_cast<double2*>(a), alpha, reinterpret_cast<const double2*>(b), beta);
+  else
+    k_masked_add<<<(int)(((int64_t)A.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
+        A.nnz, m.partner.p, A.nb_elem.p, B.nb_elem.p, A.nb_row.p, A.nb_cover.p, S.dg.prim_nsf.p, S.dg.cover_nsf.p, a, alpha,
+        b, beta);
   S.launches++;
   CQ_CUDA(cudaGetLastError());
 }
@@ -286,8 +368,12 @@ void dev_transpose(System& S, int r, const double* a, double* at) {
   RangeIndex& R = *S.ranges[r];
   CQ_CHECK(a != at, CQ_ERR_ARG, "transpose cannot run in place");
   if (R.nnz == 0) return;
-  k_transpose<<<(int)(((int64_t)R.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
-      R.nnz, R.trans_dest.p, R.nb_elem.p, R.nb_row.p, R.nb_cover.p, S.dg.prim_nsf.p, S.dg.cover_nsf.p, a, at);
+  if (S.uniform_nsf == 4 && ((uintptr_t)a | (uintptr_t)at) % 16 == 0)
+    k_transpose_nd4<<<grid_for((int64_t)R.nnz * 8), kT, 0, S.stream>>>(
+        R.nnz, R.trans_dest.p, reinterpret_cast<const double2*>(a), reinterpret_cast<double2*>(at));
+  else
+    k_transpose<<<(int)(((int64_t)R.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
+        R.nnz, R.trans_dest.p, R.nb_elem.p, R.nb_row.p, R.nb_cover.p, S.dg.prim_nsf.p, S.dg.cover_nsf.p, a, at);
   S.launches++;
   CQ_CUDA(cudaGetLastError());
 }
@@ -316,26 +402,28 @@ double acc192_to_double(const uint64_t in[3], int lsb_exp) {
   return neg ? -v : v;
 }
 
-// Grid of the exact sums: integer accumulation is associative, so the grid only sets the
-// parallelism (about four elements per thread, at most 148 SMs x 8 blocks).
+// Grid of an exact sum: integer accumulation is associative, so the grid only sets the
+// parallelism (about four elements per thread, at most 148 SMs x 4 blocks).
 static int acc_grid(int64_t n) {
   int64_t g = (n + 4 * kT - 1) / (4 * kT);
   return (int)std::max<int64_t>(1, std::min<int64_t>(g, kRedBlocks));
 }
 
-// Enqueue the three passes; the 4-word result (3 fixed-point words, flags) lands in res.
-static void exact_sum_enqueue(System& S, const double* x, const double* y, int64_t n, int* flags, uint64_t* part,
-                              uint64_t* res) {
-  const int g = acc_grid(n);
-  CQ_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(int), S.stream));
-  k_acc_emax<<<g, kT, 0, S.stream>>>(x, y, n, flags, flags + 1);
-  k_acc_sum<<<g, kT, 0, S.stream>>>(x, y, n, flags, part);
-  k_acc_final<<<1, kT, 0, S.stream>>>(part, g, flags, res);
-  S.launches += 3;
+// Enqueue the two passes of up to kSumSlots sums; the 4-word results (3 fixed-point words, flags) land in res.
+static void exact_sums_launch(int count, const double* const* x, const double* const* y, const int64_t* n, int* flags,
+                              uint64_t* part, uint64_t* res, cudaStream_t st) {
+  SumArgs A;
+  int grid = 1;
+  for (int k = 0; k < count; ++k) {
+    A.x[k] = x[k]; A.y[k] = y ? y[k] : nullptr; A.n[k] = n[k]; A.blocks[k] = acc_grid(n[k]);
+    grid = std::max(grid, A.blocks[k]);
+  }
+  k_acc_emax<<<dim3(grid, count), kT, 0, st>>>(A, flags);
+  k_acc_sum<<<dim3(grid, count), kT, 0, st>>>(A, flags, part, 3 * kRedBlocks, res);
   CQ_CUDA(cudaGetLastError());
 }
 
-// Value of a 4-word exact-sum result (k_acc_final layout).
+// Value of a 4-word exact-sum result (k_acc_sum layout).
 static double exact_sum_value(const uint64_t r[4]) {
   const int eb = (int)(uint32_t)(r[3] & 0xffffffffu);
   if ((r[3] >> 32) != 0) return std::numeric_limits<double>::quiet_NaN();
@@ -343,21 +431,15 @@ static double exact_sum_value(const uint64_t r[4]) {
   return acc192_to_double(r, eb - kEBias - kAccFrac);
 }
 
-// Scratch of the exact sums: the block partials of the sum being computed (the three passes of
-// one sum run back to back on the stream, so consecutive sums share them), then one 4-word
-// result per slot; two flag words per slot.
+// Scratch of the exact sums: the block partials of every sum of a call (kept: the calls of a system follow one
+// another on its stream) and the flags, zero between calls.
 static void acc_scratch(System& S) {
-  if (S.acc_part.n < (size_t)(3 * kRedBlocks + 4 * kSumSlots)) S.acc_part.alloc(3 * kRedBlocks + 4 * kSumSlots, S.stream);
-  if (S.acc_flags.n < (size_t)(2 * kSumSlots)) S.acc_flags.alloc(2 * kSumSlots, S.stream);
-}
-
-static double exact_sum(System& S, const double* x, const double* y, int64_t n) {
-  acc_scratch(S);
-  exact_sum_enqueue(S, x, y, n, S.acc_flags.p, S.acc_part.p, S.acc_part.p + 3 * kRedBlocks);
-  uint64_t w[4];
-  CQ_CUDA(cudaMemcpyAsync(w, S.acc_part.p + 3 * kRedBlocks, sizeof(w), cudaMemcpyDeviceToHost, S.stream));
-  host_wait(S);
-  return exact_sum_value(w);
+  if (S.acc_part.n == 0) {
+    S.acc_part.alloc((size_t)3 * kRedBlocks * kSumSlots, S.stream);
+    S.acc_flags.alloc(kSumFlags * kSumSlots, S.stream);
+    CQ_CUDA(cudaMemsetAsync(S.acc_flags.p, 0, sizeof(int) * kSumFlags * kSumSlots, S.stream));
+  }
+  if (!S.host_res) S.host_res = pinned_get();
 }
 
 void dev_dots_enqueue(System& S, int count, const double* const* x, const double* const* y, const int64_t* n) {
@@ -365,10 +447,8 @@ void dev_dots_enqueue(System& S, int count, const double* const* x, const double
   if (count == 0) return;
   acc_scratch(S);
   static_assert(4 * kSumSlots <= kPinnedWords, "pinned result buffer too small");
-  if (!S.host_res) S.host_res = pinned_get();
-  uint64_t* res = S.acc_part.p + 3 * kRedBlocks;
-  for (int k = 0; k < count; ++k) exact_sum_enqueue(S, x[k], y[k], n[k], S.acc_flags.p + 2 * k, S.acc_part.p, res + 4 * k);
-  CQ_CUDA(cudaMemcpyAsync(S.host_res, res, sizeof(uint64_t) * 4 * count, cudaMemcpyDeviceToHost, S.stream));
+  exact_sums_launch(count, x, y, n, S.acc_flags.p, S.acc_part.p, S.host_res, S.stream);
+  S.launches += 2;
 }
 
 void dev_dots_fetch(System& S, int count, double* out) {
@@ -382,7 +462,11 @@ void dev_dots(System& S, int count, const double* const* x, const double* const*
   dev_dots_fetch(S, count, out);
 }
 
-double dev_dot(System& S, const double* x, const double* y, int64_t n) { return exact_sum(S, x, y, n); }
+double dev_dot(System& S, const double* x, const double* y, int64_t n) {
+  double v = 0.0;
+  dev_dots(S, 1, &x, &y, &n, &v);
+  return v;
+}
 
 double dev_trace(System& S, int r, const double* a) {
   RangeIndex& R = *S.ranges[r];
@@ -396,7 +480,7 @@ double dev_trace(System& S, int r, const double* a) {
   k_gather_diag<<<(N + kT - 1) / kT, kT, 0, S.stream>>>(N, R.onsite.p, S.dg.prim_nsf.p, S.diag_off.p, a, S.diag_buf.p);
   S.launches++;
   CQ_CUDA(cudaGetLastError());
-  return exact_sum(S, S.diag_buf.p, nullptr, (int64_t)S.diag_buf.n);
+  return dev_dot(S, S.diag_buf.p, nullptr, (int64_t)S.diag_buf.n);
 }
 void dev_set_onsite_diag(System& S, int r, double* a, double value) {
   RangeIndex& R = *S.ranges[r];
@@ -429,16 +513,18 @@ void dev_h_limits(System& S, int r, const double* h, double* hmin, double* hmax)
 // Some callers cannot allocate device memory at the moment they need a trace: a Fortran/MPI
 // host that has given the whole device to its own memory pool, or a latency-critical loop that
 // must not take the device-wide synchronisation cudaMalloc and cudaFree can imply.  This entry
-// point runs the same three kernels as the library's traces, with their scratch (block
+// point runs the same two kernels as the library's traces, with their scratch (block
 // partials, results and flags) in one static device array instead of library-allocated memory.
 // Every call uses that same array, so calls that overlap on the GPU (from two streams or two
 // threads) race on it.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kNoAllocSums = CQ_NOALLOC_MAX_SUMS;
-// words: block partials of one sum | 4-word result per sum | 2 int flags per sum (one word)
-constexpr int kNoAllocWords = 3 * kRedBlocks + 4 * kNoAllocSums + kNoAllocSums;
-static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];   // 28.7 KiB per device
+// words: block partials of two sums | 4-word result per sum | 3 int flags per sum
+constexpr int kNoAllocPairs = 2;                                   // sums whose passes share two launches
+constexpr int kNoAllocFlags = (kSumFlags * kNoAllocSums + 1) / 2;   // words
+constexpr int kNoAllocWords = 3 * kRedBlocks * kNoAllocPairs + 4 * kNoAllocSums + kNoAllocFlags;
+static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];   // 28.1 KiB per device
 
 // Device address of the static scratch on the current device.  The host-side name of the array
 // is not a device address, so it is looked up with cudaGetSymbolAddress on every call (cheap, and
@@ -466,20 +552,14 @@ extern "C" int cq_exact_dots_noalloc(int count, const double* const* x_dev, cons
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint64_t* base = noalloc_scratch();
     uint64_t* part = base;
-    uint64_t* res = base + 3 * kRedBlocks;
-    int* flags = reinterpret_cast<int*>(base + 3 * kRedBlocks + 4 * kNoAllocSums);
-    // the pass-1 flags (largest exponent, non-finite) start at zero; the partials and results
+    uint64_t* res = base + 3 * kRedBlocks * kNoAllocPairs;
+    int* flags = reinterpret_cast<int*>(res + 4 * kNoAllocSums);
+    // the flags (largest exponent, non-finite, blocks done) start at zero; the partials and results
     // are overwritten by every call
-    CQ_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 2 * count, st));
-    for (int k = 0; k < count; ++k) {
-      const double* x = x_dev[k];
-      const double* y = y_dev ? y_dev[k] : nullptr;
-      const int g = acc_grid(n[k]);
-      k_acc_emax<<<g, kT, 0, st>>>(x, y, n[k], flags + 2 * k, flags + 2 * k + 1);
-      k_acc_sum<<<g, kT, 0, st>>>(x, y, n[k], flags + 2 * k, part);
-      k_acc_final<<<1, kT, 0, st>>>(part, g, flags + 2 * k, res + 4 * k);
-    }
-    CQ_CUDA(cudaGetLastError());
+    CQ_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * kSumFlags * count, st));
+    for (int k = 0; k < count; k += kNoAllocPairs)
+      exact_sums_launch(std::min(kNoAllocPairs, count - k), x_dev + k, y_dev ? y_dev + k : nullptr, n + k,
+                        flags + kSumFlags * k, part, res + 4 * k, st);
     uint64_t w[4 * kNoAllocSums];
     CQ_CUDA(cudaMemcpyAsync(w, res, sizeof(uint64_t) * 4 * count, cudaMemcpyDeviceToHost, st));
     CQ_CUDA(cudaStreamSynchronize(st));

@@ -124,6 +124,17 @@ System& system_of(cq_system* s) {
 int guarded_call(const std::function<void()>& f) { return guarded(f); }
 }  // namespace cqb
 
+// a = alpha a + beta b: one pass, the roundings of scale then axpy; two passes where b overlaps a (the reference's
+// second step then reads what its first has written)
+static void sum_same_range(System& S, double* a, double alpha, const double* b, double beta, int64_t n) {
+  if (a + n <= b || b + n <= a) {
+    dev_axpby(S, a, n, alpha, beta, b);
+  } else {
+    dev_scale(S, a, n, alpha);
+    dev_axpy(S, a, n, beta, b);
+  }
+}
+
 static void check_sys(cq_system* s) { CQ_CHECK(s != nullptr, CQ_ERR_ARG, "null system"); }
 static void check_range(cq_system* s, int r) {
   CQ_CHECK(r >= 0 && r < (int)s->S.ranges.size(), CQ_ERR_ARG, "range index out of bounds");
@@ -336,8 +347,7 @@ int cq_matrix_sum(cq_system* sys, int ra, double* a_dev, double alpha, int rb, c
     check_sys(sys); check_range(sys, ra); check_range(sys, rb);
     System& S = sys->S;
     if (ra == rb) {
-      dev_scale(S, a_dev, S.ranges[ra]->length, alpha);
-      dev_axpy(S, a_dev, S.ranges[ra]->length, beta, b_dev);
+      sum_same_range(S, a_dev, alpha, b_dev, beta, S.ranges[ra]->length);
     } else {
       dev_matrix_add(S, ra, a_dev, alpha, rb, b_dev, beta);
     }
@@ -764,8 +774,7 @@ int cq_matrix_sum_id(cq_system* sys, int ida, double alpha, int idb, double beta
     BoundMatrix &A = bound(sys, ida), &B = bound(sys, idb);
     System& S = sys->S;
     if (A.r == B.r) {
-      dev_scale(S, A.dev.p, S.ranges[A.r]->length, alpha);
-      dev_axpy(S, A.dev.p, S.ranges[A.r]->length, beta, B.dev.p);
+      sum_same_range(S, A.dev.p, alpha, B.dev.p, beta, S.ranges[A.r]->length);
     } else {
       dev_matrix_add(S, A.r, A.dev.p, alpha, B.r, B.dev.p, beta);
     }

@@ -420,7 +420,7 @@ int cq_lnv_solve_host(cq_lnv* s, const double* S, const double* H, double* L_out
  * bit-identical to it.  x_dev / y_dev are host arrays of device pointers; work is enqueued on
  * `stream` (a cudaStream_t, NULL = the default stream) and the call synchronises it.
  *   - At most CQ_NOALLOC_MAX_SUMS sums per call; more is rejected with CQ_ERR_ARG.
- *   - The scratch is one static device array of 28.7 KiB that every GPU loading the library
+ *   - The scratch is one static device array of 28.1 KiB that every GPU loading the library
  *     holds until exit.  Every call looks up that array's device address on the current device
  *     (the first lookup on a device may load the library's device code there: make the first
  *     call before any stream capture on that device).

@@ -79,3 +79,68 @@ def test_4x4_kernels_give_the_same_bits(shape, exact):
             g.synchronize()
             ref = ops[out].clone() if ref is None else ref
             assert torch.equal(ops[out], ref), (t, rc, v)
+
+
+@pytest.mark.parametrize("nd", ["4", "13", "4_13"])
+def test_transpose_and_sums_against_index_arithmetic(nd):
+    """Transposes and sums of equal and different ranges, element by element: 4 x 4 blocks (aligned, then on an odd
+    8-byte boundary), 13 x 13 and both; a sum with itself keeps the two steps of the reference (scale, then add)."""
+    import torch
+    import cq_b200
+    coords, cell = inputs.si_cluster(37, sigma=0.1, seed=61)
+    nsf = np.array([{"4": 4, "13": 13, "4_13": 13 if k % 3 == 0 else 4}[nd] for k in range(len(coords))], np.int32)
+    g = cq_b200.System(coords, cell, nsf, [9.0, 13.0])
+    bls = [g.blocklist(r, coords, cell) for r in range(2)]
+    vals = [inputs.random_blocks(bls[r], 3 + r, inputs.TAG_RANDOM_A) for r in range(2)]
+    short, wide = bm.block_dict(bls[0]), bm.block_dict(bls[1])
+    for shift in (0, 1):
+        dev = []
+        for v in vals + [np.zeros(bls[0].length)]:
+            t = torch.zeros(len(v) + 1, dtype=torch.float64, device="cuda")
+            t[shift:shift + len(v)] = torch.from_numpy(v)
+            dev.append(t[shift:shift + len(v)])
+        a, b, at = dev
+        torch.cuda.synchronize()
+        g.transpose(0, a, at)
+        g.synchronize()
+        assert np.array_equal(at.cpu().numpy(), bm.kat_transpose(bls[0], vals[0]))
+        g.matrix_sum(0, a, 0.5, 0, at, -3.0)
+        g.synchronize()
+        want = vals[0] * 0.5 + -3.0 * bm.kat_transpose(bls[0], vals[0])
+        assert np.array_equal(a.cpu().numpy(), want)
+        g.matrix_sum(0, a, 2.0, 0, a, 0.25)                   # b is a: fl(2a), then fl(2a) + fl(0.25 fl(2a))
+        g.synchronize()
+        want = want * 2.0 + 0.25 * (want * 2.0)
+        assert np.array_equal(a.cpu().numpy(), want)
+        g.matrix_sum(1, b, 1.5, 0, at, 0.75)                  # the wider range keeps its other blocks
+        g.synchronize()
+        want_b, t = vals[1].copy(), bm.kat_transpose(bls[0], vals[0])
+        for key, (off, ni, nj) in short.items():
+            o = wide[key][0]
+            want_b[o:o + ni * nj] = 1.5 * vals[1][o:o + ni * nj] + 0.75 * t[off:off + ni * nj]
+        assert np.array_equal(b.cpu().numpy(), want_b)
+
+
+def test_exact_sums_of_extreme_terms():
+    """Traces with subnormal and huge terms, both signs, cancelling sums, zeros, infinities and NaN: the exact sum
+    rounded once (Fractions of the rounded products; terms below 2^-150 of the largest do not occur)."""
+    import fractions
+    import torch
+    import cq_b200
+    g = cq_b200.System(*inputs.si_cluster(5, sigma=0.1, seed=71), np.full(5, 4, np.int32), [9.0])
+    n = g.length(0)
+    rng = np.random.default_rng(8)
+    cases = [np.where(rng.random(n) < 0.5, 5e-324, -3e-310), rng.standard_normal(n) * 2.0 ** rng.integers(-40, 40, n),
+             rng.standard_normal(n) * 1e300, np.zeros(n)]
+    one = torch.ones(n, dtype=torch.float64, device="cuda")
+    for x in cases:
+        d = torch.from_numpy(x).cuda()
+        torch.cuda.synchronize()
+        want = float(sum((fractions.Fraction(float(v)) for v in x), fractions.Fraction(0)))
+        assert g.product_trace(0, d, one) == want
+        assert cq_b200.exact_dots_noalloc([d] * 3, [one, None, one]) == [want] * 3
+    for bad in (np.inf, np.nan):
+        d = torch.from_numpy(np.where(np.arange(n) == n - 1, bad, 1.0)).cuda()
+        torch.cuda.synchronize()
+        assert np.isnan(g.product_trace(0, d, one))
+        assert g.product_trace(0, one, one) == n              # the flags of the last sum are cleared
