@@ -676,96 +676,6 @@ __global__ void __launch_bounds__(128) k_mult_nd4_quad(MultArgs M, const int* __
   }
 }
 
-// FP64 on the tensor cores (DMMA, mma.sync.m8n8k4.f64): one warp per output block, the block padded to
-// 16 x 16 as 2 x 2 tiles of 8 x 8, the contraction in steps of 4.  Per step a lane loads one element of
-// each first-operand row tile (row g = lane / 4, column t = lane % 4 of the step) and one of each B column
-// tile (row t, column g) straight from the block storage (zeros outside the blocks), and the warp issues
-// four MMAs; C/D hold rows g, columns 2t and 2t + 1 of each tile.  The terms of an element are summed in
-// FP64 by the tensor cores in the blocks' order, four at a time, so the result differs from the reference
-// kernel's separate multiply and add in rounding only (about 1e-16 of sum |a||b|).
-__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
-// One term's operands in DMMA fragment order: for k-step ks (contraction columns 4 ks .. 4 ks + 3) a
-// lane holds element (row 8 i + g, column 4 ks + t) of the first operand for row tile i and element
-// (row 4 ks + t, column 8 j + g) of the B operand for column tile j; zeros outside the blocks.
-template <int TYPE>
-__device__ __forceinline__ void dmma_load_term(const MultArgs& M, int2 pr, int ndi, int ndo, int g, int t,
-                                               double (&av)[4][2], double (&bv)[4][2], int& nks) {
-  const double* X = M.x + M.x_elem[pr.x];
-  const double* B = M.b + M.b_elem[pr.y];
-  const int ndk = TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]];
-  nks = (ndk + 3) >> 2;
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    const int kk = 4 * ks + t;
-    const bool kin = kk < ndk;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = 8 * i + g;
-      av[ks][i] = (kin && r < ndi) ? __ldg(X + r + ndi * kk) : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int c = 8 * j + g;
-      // type 1: B(kk, c) of the nd_k x nd_j block; type 2: B(c, kk) of the nd_k x nd_j block (B^T)
-      bv[ks][j] = (kin && c < ndo) ? __ldg(TYPE == 1 ? B + kk + ndk * c : B + c + ndo * kk) : 0.0;
-    }
-  }
-}
-
-// The next term's operands are loaded while the current term's MMAs run.
-template <int TYPE>
-__global__ void __launch_bounds__(128) k_mult_dmma(MultArgs M) {
-  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= M.n_out) return;
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int ndi = M.prim_nsf[M.o_row[q]];
-  const int ndo = M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
-  const int nrt = ndi > 8 ? 2 : 1, nct = ndo > 8 ? 2 : 1;
-  double acc[2][2][2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) { acc[i][j][0] = 0.0; acc[i][j][1] = 0.0; }
-  const int64_t p0 = M.ptr[q], p1 = M.ptr[q + 1];
-  double av[4][2], bv[4][2];
-  int nks = 0;
-  if (p0 < p1) dmma_load_term<TYPE>(M, __ldcs(M.pairs + p0), ndi, ndo, g, t, av, bv, nks);
-  for (int64_t p = p0; p < p1; ++p) {
-    double nav[4][2], nbv[4][2];
-    int nnks = 0;
-    if (p + 1 < p1) dmma_load_term<TYPE>(M, __ldcs(M.pairs + p + 1), ndi, ndo, g, t, nav, nbv, nnks);
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-      if (ks < nks) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            if (i < nrt && j < nct) dmma_8x8x4(acc[i][j], av[ks][i], bv[ks][j]);
-      }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) { av[ks][i] = nav[ks][i]; bv[ks][i] = nbv[ks][i]; }
-    nks = nnks;
-  }
-  double* O = M.out + M.o_elem[q];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = 8 * i + g, c = 8 * j + 2 * t + e;
-        if (r < ndi && c < ndo) O[r + ndi * c] = acc[i][j][e];
-      }
-}
-
 // Any block sizes up to 16 (DZP 13 x 13, mixed SZ/DZP): LPB lanes per output block (8: four blocks per warp,
 // lane l owns columns l and l + 8; 16: two blocks per warp, one column per lane), every row of those columns in
 // the lane's registers.  The group stages the two operand blocks of a pair in shared memory with cp.async; X
@@ -978,6 +888,116 @@ __global__ void __launch_bounds__(64) k_mult_group(MultArgs M, const int* __rest
   const int base = (blockIdx.x * 2 + warp) * Q::kBlocks;
   if (base >= M.n_out) return;                  // whole warp
   warp_group<TYPE, EXACT, U, MAXND, LPB, STAGES>(M, order, base, group_smem + warp * Q::kWarpBytes);
+}
+
+// FP64 on the tensor cores (DMMA, mma.sync.m8n8k4.f64): one warp per output block, the block padded to 16 x 16 as
+// 2 x 2 tiles of 8 x 8.  Per step of four contraction indices a lane reads one element of each first-operand row
+// tile (row g = lane / 4, index t = lane % 4 of the step) and one of each B column tile (index t, column g), zeros
+// outside the blocks, and the warp issues four MMAs; C/D hold rows g, columns 2t and 2t + 1 of each tile.  The
+// terms of an element are summed in FP64 by the tensor cores in the blocks' order, four at a time, so the result
+// differs from the reference kernel's separate multiply and add in rounding only (about 1e-16 of sum |a||b|).
+//
+// Four pairs at a time are staged in shared memory (cp.async, eight lanes per pair) and their contractions run
+// as one: the steps cross from one pair to the next, so four 13 x 13 pairs take 13 steps instead of 4 x 4 and
+// the order of the terms stays.  What bounds it: the FP64 tensor pipe (52 MMAs per four pairs, 52 SM cycles a
+// pair), the shared-memory reads of the fragments (33 L1 wavefronts a pair and about as many to stage it) and the
+// 2.7 KB a pair moves from L2 (42 cycles).  One stage: the other warps of the SM hide its latency.
+// Measured (216-atom DZP cell, SLS = LS.S, 3.4 M pairs): 1.23 ms = 12.0 TFLOP/s, tensor pipe 50 % busy, L2 at 66 % of
+// its throughput; operands read straight from global memory, one pair at a time, 1.71 ms. The eight products of
+// an LNV call 25.1 -> 19.8 ms.
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+template <int TYPE, int U, int MAXND>
+__global__ void __launch_bounds__(64) k_mult_dmma(MultArgs M, const int* __restrict__ order) {
+  constexpr int kStride = GroupShape<MAXND, 8, 1>::kStrideB;       // bytes of one staged block
+  __shared__ __align__(128) unsigned char smem[2][8 * kStride];    // per warp: four X and four B blocks
+  const unsigned kFull = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = blockIdx.x * 2 + warp;
+  if (slot >= M.n_out) return;                    // whole warp
+  const int q = order[slot];
+  const int g = lane >> 2, t = lane & 3;          // fragment row / column and contraction index
+  const int gp = lane >> 3, l = lane & 7;         // staging: pair and lane of its group
+  unsigned char* W = smem[warp];
+  const int ndi = U > 0 ? U : M.prim_nsf[M.o_row[q]];
+  const int ndo = U > 0 ? U : M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
+  const bool r0 = U >= 8 || g < ndi, r1 = g + 8 < ndi, c0 = U >= 8 || g < ndo, c1 = g + 8 < ndo;
+  const bool rt = ndi > 8, ct = ndo > 8;          // a second row / column tile
+  double acc[2][2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int2* pairs = M.pairs + M.ptr[q];
+  const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
+  const uint32_t w0 = smem_addr(W);
+  int2 pn = gp < nt ? __ldcs(pairs + gp) : make_int2(-1, -1);      // the group's pair, loaded a round ahead
+  for (int t0 = 0; t0 < nt; t0 += 4) {
+    const int2 pr = pn;
+    pn = t0 + 4 + gp < nt ? __ldcs(pairs + t0 + 4 + gp) : make_int2(-1, -1);
+    int nk = 0;
+    bool px = false, pb = false;                  // 8-byte phases of the copies
+    if (pr.x >= 0) {
+      const double* Xg = M.x + (U > 0 ? (int64_t)pr.x * (U * U) : M.x_elem[pr.x]);
+      const double* Bg = M.b + (U > 0 ? (int64_t)pr.y * (U * U) : M.b_elem[pr.y]);
+      nk = U > 0 ? U : (TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]]);
+      px = ((uintptr_t)Xg >> 3) & 1;
+      pb = ((uintptr_t)Bg >> 3) & 1;
+      group_copy<U, 8>(w0 + gp * kStride, Xg, ndi * nk, l);
+      group_copy<U, 8>(w0 + (4 + gp) * kStride, Bg, nk * ndo, l);
+    }
+    cp_async_commit();
+    const unsigned mx = __ballot_sync(kFull, px), mb = __ballot_sync(kFull, pb);
+    // contraction offsets of the pairs
+    const int n0 = U > 0 ? U : __shfl_sync(kFull, nk, 0), n1 = U > 0 ? U : __shfl_sync(kFull, nk, 8),
+              n2 = U > 0 ? U : __shfl_sync(kFull, nk, 16), n3 = U > 0 ? U : __shfl_sync(kFull, nk, 24);
+    const int o1 = n0, o2 = o1 + n1, o3 = o2 + n2;
+    const int K = U > 0 ? U * min(4, nt - t0) : o3 + n3;
+    cp_async_wait<0>();
+    __syncwarp();
+    auto step = [&](int ks, bool all) {
+      const int kk = 4 * ks + t;
+      const int p = U > 0 ? kk / (U > 0 ? U : 1) : (kk >= o1) + (kk >= o2) + (kk >= o3);
+      const int off = U > 0 ? p * U : p == 0 ? 0 : p == 1 ? o1 : p == 2 ? o2 : o3;
+      const int n = kk - off;
+      const bool in = all || kk < K;
+      const double* X = reinterpret_cast<const double*>(W + p * kStride) + ((mx >> (8 * p)) & 1) + g + ndi * n;
+      const int np = U > 0 ? U : p == 0 ? n0 : p == 1 ? n1 : p == 2 ? n2 : n3;
+      const double* B = reinterpret_cast<const double*>(W + (4 + p) * kStride) + ((mb >> (8 * p)) & 1) +
+                        (TYPE == 1 ? n + np * g : g + ndo * n);
+      const double a0 = in && r0 ? X[0] : 0.0, a1 = in && r1 ? X[8] : 0.0;
+      const double b0 = in && c0 ? B[0] : 0.0, b1 = in && c1 ? B[TYPE == 1 ? 8 * np : 8] : 0.0;
+      dmma_8x8x4(acc[0][0], a0, b0);
+      if (ct) dmma_8x8x4(acc[0][1], a0, b1);
+      if (rt) dmma_8x8x4(acc[1][0], a1, b0);
+      if (rt && ct) dmma_8x8x4(acc[1][1], a1, b1);
+    };
+    if (U > 0 && K == 4 * U) {
+#pragma unroll
+      for (int ks = 0; ks < U; ++ks) step(ks, true);
+    } else {
+      for (int ks = 0; 4 * ks < K; ++ks) step(ks, false);
+    }
+    __syncwarp();                                 // the blocks are read before the next round replaces them
+  }
+  // results through shared memory, so that the block is written along memory
+  double* O = reinterpret_cast<double*>(W);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = 8 * i + g, c = 8 * j + 2 * t + e;
+        if (r < ndi && c < ndo) O[r + ndi * c] = acc[i][j][e];
+      }
+  __syncwarp();
+  double* D = M.out + (U > 0 ? (int64_t)q * (U * U) : M.o_elem[q]);
+  for (int e = lane; e < ndi * ndo; e += 32) __stcs(D + e, O[e]);
 }
 
 // Many independent products in one persistent launch (the concatenation of their output-block
@@ -1355,9 +1375,15 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   // those of the CUDA-core kernels (checked on B200), about three times faster on 13 x 13 blocks
   // (unless a CUDA-core variant is forced with CQ_OPT_MULT_VARIANT)
   if (exact == kPrecFp64Tensor || (exact == 0 && S.max_nsf > 8 && S.mult_variant == kVariantAuto)) {
-    const int grid = (M.n_out * 32 + 127) / 128;
-    if (P.mult_type == 1) k_mult_dmma<1><<<grid, 128, 0, st>>>(M);
-    else k_mult_dmma<2><<<grid, 128, 0, st>>>(M);
+    ensure_order(S, P);
+    const int grid = (M.n_out + 1) / 2;
+    if (P.mult_type == 1) {
+      if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
+      else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
+    } else {
+      if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
+      else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
+    }
     S.launches++;
     CQ_CUDA(cudaGetLastError());
   } else {
