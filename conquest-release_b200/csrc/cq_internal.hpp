@@ -214,22 +214,15 @@ struct ProductPlan {
   float tune_ms[7] = {0, 0, 0, 0, 0, 0, 0};
 };
 
-// Split-precision tensor-core product: pair lists sorted by the first operand block,
-// and groups of consecutive output blocks of one row (one warp each).
+// Split-precision tensor-core product: pair lists sorted by the first operand block (one warp per output block).
 struct MixedPlan {
   int mult_type = 1, ra = -1, rb = -1, rc = -1, out_range = -1;
-  int n_groups[4] = {-1, -1, -1, -1};   // groups of 1, 2, 4 and 8 output blocks (-1: not built yet)
-  int tuned_g = -1;                 // group size chosen by the autotuner (index into 1, 2, 4, 8)
   int kernel = -1;                  // 0 = tcgen05 tiles, 1 = per-block mma.sync (-1: not chosen yet)
-  float tune_ms[4] = {0, 0, 0, 0};
-  int tuned_g6 = -1;                // three-part split: group size chosen (index into 1, 2, 4)
-  float tune_ms6[3] = {0, 0, 0};
   int64_t n_pairs = 0, flops = 0;
   DevBuf<int64_t> own_ptr;        // type 2 only (type 1 uses the FP64 plan's lists, already sorted)
   DevBuf<int2> own_pairs;
   const int64_t* ptr = nullptr;
   const int2* pairs = nullptr;
-  DevBuf<int2> groups[4];
 };
 
 struct FragBuf { DevBuf<uint4> hi, lo, mid; };   // mid: three-part split only
@@ -302,7 +295,6 @@ struct System {
   int mixed_kernel = -1;          // split-precision products: 0 = tcgen05 tiles (umma.cu), 1 = mma.sync per block,
                                   // -1 = chosen per product by the tile plan's useful fraction
   int* umma_err_host = nullptr;   // mapped host word set by a tensor-core product whose bounded wait ran out
-  int split_group = -1;           // CQ_OPT_SPLIT_GROUP: forced output blocks per mma.sync split warp (-1 tuned)
   int umma_test_stall = 0;        // test hook (CQ_OPT_TEST_STALL): the next tensor-core product stalls
   int* umma_err_dev = nullptr;
   cudaStream_t stream = nullptr;  // the stream all work of the system is enqueued on
@@ -367,8 +359,6 @@ void generate_SH(System& S, int r, int which, uint64_t seed, double* out);
 
 // mixed.cu
 void to_fragments(System& S, int r, const double* src, int role_b, int trans, uint4* hi, uint4* lo, uint4* mid);
-void launch_mult_tc(System& S, MixedPlan& MP, const uint4* xa_hi, const uint4* xa_lo, const uint4* bb_hi,
-                    const uint4* bb_lo, double* out);
 // split-precision mat_mult with the roles of launch_mat_mult: tcgen05 tiles where every block size is
 // 4..128 (unless the system selects the per-block kernel), else the per-block mma.sync kernel
 // `exact` argument of launch_mat_mult: 1 = the reference kernel's separate multiply and add, 0 = fused

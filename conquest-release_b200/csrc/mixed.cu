@@ -7,22 +7,15 @@
 // six MMAs per term, FP64 accumulation across terms) carries about 22.  The result is written back as FP64 into
 // the block storage of the output range, so the matrices of the chain stay FP64.
 //
-// Work decomposition (output stationary, same pair lists as the FP64 path):
-// one warp owns G consecutive output blocks of one output row i (G = 1, 2, 4 or 8, chosen per
-// product by the autotuner: larger groups reuse each first-operand fragment more, smaller ones
-// need fewer registers and give more warps; the results do not depend on G, since each output
-// block accumulates its own pairs in its own order).  Their pair
-// lists are sorted by the first operand block (A_ik for type 1, C_ij for type 2,
-// both in row i), so the warp walks the union of those blocks in order, loads each
-// first-operand fragment once and multiplies it into every output block whose list
-// contains it.  Operands are pre-converted into the per-lane fragment order of
-// mma.m16n8k16, so every fragment is one coalesced 16-byte load per lane.
+// Work decomposition (output stationary): one warp owns one output block and takes the terms of its pair list,
+// sorted by the first operand block (A_ik for type 1, C_ij for type 2), in order.  Operands are pre-converted
+// into the per-lane fragment order of mma.m16n8k16, so every fragment is one coalesced 16-byte load per lane.
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <climits>
 
 #include "cq_internal.hpp"
+
 
 namespace cqb {
 namespace {
@@ -108,8 +101,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, uint32_t
 }
 
 struct TCArgs {
-  const int2* __restrict__ groups;     // (first output block, count) per warp, never crossing a row
-  int n_groups;
+  int n_out;
   const int64_t* __restrict__ ptr;     // pair list offsets per output block
   const int2* __restrict__ pairs;      // (first-operand block, B block), first operand ascending
   const uint4* __restrict__ xa_hi;     // first operand, A-role fragments
@@ -126,178 +118,9 @@ struct TCArgs {
   double* __restrict__ out;
 };
 
-template <int kG>   // output blocks per warp
-__global__ void __launch_bounds__(128) k_mult_tc(TCArgs M) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= M.n_groups) return;
-  const int2 grp = M.groups[w];
-  int64_t p[kG], pe[kG];
-  int nx[kG];
-  float acc[kG][2][4];
-#pragma unroll
-  for (int b = 0; b < kG; ++b) {
-    if (b < grp.y) { p[b] = M.ptr[grp.x + b]; pe[b] = M.ptr[grp.x + b + 1]; }
-    else { p[b] = 0; pe[b] = 0; }
-    nx[b] = p[b] < pe[b] ? M.pairs[p[b]].x : INT_MAX;
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[b][h][r] = 0.f;
-  }
-  while (true) {
-    int kc = INT_MAX;
-#pragma unroll
-    for (int b = 0; b < kG; ++b) kc = min(kc, nx[b]);
-    if (kc == INT_MAX) break;
-    const uint4 ah = __ldg(M.xa_hi + (int64_t)kc * 32 + lane);
-    const uint4 al = __ldg(M.xa_lo + (int64_t)kc * 32 + lane);
-#pragma unroll
-    for (int b = 0; b < kG; ++b) {
-      if (nx[b] == kc) {
-        const int y = M.pairs[p[b]].y;
-        const uint4 bh = __ldg(M.bb_hi + (int64_t)y * 32 + lane);
-        const uint4 bl = __ldg(M.bb_lo + (int64_t)y * 32 + lane);
-        mma_bf16(acc[b][0], al, bh.x, bh.y);
-        mma_bf16(acc[b][0], ah, bl.x, bl.y);
-        mma_bf16(acc[b][0], ah, bh.x, bh.y);
-        mma_bf16(acc[b][1], al, bh.z, bh.w);
-        mma_bf16(acc[b][1], ah, bl.z, bl.w);
-        mma_bf16(acc[b][1], ah, bh.z, bh.w);
-        ++p[b];
-        nx[b] = p[b] < pe[b] ? M.pairs[p[b]].x : INT_MAX;
-      }
-    }
-  }
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int b = 0; b < kG; ++b) {
-    if (b < grp.y) {
-      const int q = grp.x + b;
-      const int ndr = M.prim_nsf[M.o_row[q]], ndc = M.cover_nsf[M.o_cover[q]];
-      double* O = M.out + M.o_elem[q];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          int row = g + ((r & 2) ? 8 : 0), col = 8 * h + 2 * t + (r & 1);
-          if (row < ndr && col < ndc) O[row + ndr * col] = (double)acc[b][h][r];
-        }
-    }
-  }
-}
-
-// One output block per warp with the next term's four fragments loaded while the current term's
-// six MMAs run (the group-of-one case of k_mult_tc, same terms in the same order, so the same
-// result): the fragment loads of consecutive terms overlap instead of stalling each term.
-__global__ void __launch_bounds__(128) k_mult_tc1(TCArgs M) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= M.n_groups) return;
-  const int q = M.groups[w].x;
-  int64_t p = M.ptr[q];
-  const int64_t pe = M.ptr[q + 1];
-  float acc[2][4];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) acc[h][r] = 0.f;
-  uint4 ah = {0, 0, 0, 0}, al = ah, bh = ah, bl = ah;
-  if (p < pe) {
-    const int2 pr = M.pairs[p];
-    ah = __ldg(M.xa_hi + (int64_t)pr.x * 32 + lane);
-    al = __ldg(M.xa_lo + (int64_t)pr.x * 32 + lane);
-    bh = __ldg(M.bb_hi + (int64_t)pr.y * 32 + lane);
-    bl = __ldg(M.bb_lo + (int64_t)pr.y * 32 + lane);
-  }
-  for (; p < pe; ++p) {
-    uint4 nah = ah, nal = al, nbh = bh, nbl = bl;
-    if (p + 1 < pe) {
-      const int2 pn = M.pairs[p + 1];
-      nah = __ldg(M.xa_hi + (int64_t)pn.x * 32 + lane);
-      nal = __ldg(M.xa_lo + (int64_t)pn.x * 32 + lane);
-      nbh = __ldg(M.bb_hi + (int64_t)pn.y * 32 + lane);
-      nbl = __ldg(M.bb_lo + (int64_t)pn.y * 32 + lane);
-    }
-    mma_bf16(acc[0], al, bh.x, bh.y);
-    mma_bf16(acc[0], ah, bl.x, bl.y);
-    mma_bf16(acc[0], ah, bh.x, bh.y);
-    mma_bf16(acc[1], al, bh.z, bh.w);
-    mma_bf16(acc[1], ah, bl.z, bl.w);
-    mma_bf16(acc[1], ah, bh.z, bh.w);
-    ah = nah; al = nal; bh = nbh; bl = nbl;
-  }
-  const int g = lane >> 2, t = lane & 3;
-  const int ndr = M.prim_nsf[M.o_row[q]], ndc = M.cover_nsf[M.o_cover[q]];
-  double* O = M.out + M.o_elem[q];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      int row = g + ((r & 2) ? 8 : 0), col = 8 * h + 2 * t + (r & 1);
-      if (row < ndr && col < ndc) O[row + ndr * col] = (double)acc[h][r];
-    }
-}
-
-// Three-part split (BF16x6): v = hi + mid + lo, one output block per warp.  Per term and n8 half the
-// six products that carry terms down to 2^-16 of hi.hi run into a zeroed FP32 accumulator, smallest
-// first (hi.lo, lo.hi, mid.mid, hi.mid, mid.hi, hi.hi), and the term's 16 x 8 result is added to FP64
-// accumulators, so the FP32 rounding spans one 16-wide contraction rather than the whole sum.  The
-// omitted products (mid.lo, lo.mid, lo.lo) and the split remainders are below 2^-23 of |a||b| per
-// element product.  The next term's six fragments load while the current term's MMAs run.
-__global__ void __launch_bounds__(128) k_mult_tc6(TCArgs M) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= M.n_groups) return;
-  const int q = M.groups[w].x;
-  int64_t p = M.ptr[q];
-  const int64_t pe = M.ptr[q + 1];
-  double acc[2][4];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) acc[h][r] = 0.0;
-  uint4 ah = {0, 0, 0, 0}, am = ah, al = ah, bh = ah, bm = ah, bl = ah;
-  if (p < pe) {
-    const int2 pr = M.pairs[p];
-    ah = __ldg(M.xa_hi + (int64_t)pr.x * 32 + lane);
-    am = __ldg(M.xa_mid + (int64_t)pr.x * 32 + lane);
-    al = __ldg(M.xa_lo + (int64_t)pr.x * 32 + lane);
-    bh = __ldg(M.bb_hi + (int64_t)pr.y * 32 + lane);
-    bm = __ldg(M.bb_mid + (int64_t)pr.y * 32 + lane);
-    bl = __ldg(M.bb_lo + (int64_t)pr.y * 32 + lane);
-  }
-  for (; p < pe; ++p) {
-    uint4 nah = ah, nam = am, nal = al, nbh = bh, nbm = bm, nbl = bl;
-    if (p + 1 < pe) {
-      const int2 pn = M.pairs[p + 1];
-      nah = __ldg(M.xa_hi + (int64_t)pn.x * 32 + lane);
-      nam = __ldg(M.xa_mid + (int64_t)pn.x * 32 + lane);
-      nal = __ldg(M.xa_lo + (int64_t)pn.x * 32 + lane);
-      nbh = __ldg(M.bb_hi + (int64_t)pn.y * 32 + lane);
-      nbm = __ldg(M.bb_mid + (int64_t)pn.y * 32 + lane);
-      nbl = __ldg(M.bb_lo + (int64_t)pn.y * 32 + lane);
-    }
-    float t[2][4];
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) t[h][r] = 0.f;
-    mma_bf16(t[0], ah, bl.x, bl.y);
-    mma_bf16(t[0], al, bh.x, bh.y);
-    mma_bf16(t[0], am, bm.x, bm.y);
-    mma_bf16(t[0], ah, bm.x, bm.y);
-    mma_bf16(t[0], am, bh.x, bh.y);
-    mma_bf16(t[0], ah, bh.x, bh.y);
-    mma_bf16(t[1], ah, bl.z, bl.w);
-    mma_bf16(t[1], al, bh.z, bh.w);
-    mma_bf16(t[1], am, bm.z, bm.w);
-    mma_bf16(t[1], ah, bm.z, bm.w);
-    mma_bf16(t[1], am, bh.z, bh.w);
-    mma_bf16(t[1], ah, bh.z, bh.w);
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[h][r] += (double)t[h][r];
-    ah = nah; am = nam; al = nal; bh = nbh; bm = nbm; bl = nbl;
-  }
+// the accumulators (rows g and g + 8, columns 2 t4 and 2 t4 + 1 of each n8 half) to output block q
+template <class Acc>
+__device__ __forceinline__ void store_block(const TCArgs& M, int q, int lane, const Acc (&acc)[2][4]) {
   const int g = lane >> 2, t4 = lane & 3;
   const int ndr = M.prim_nsf[M.o_row[q]], ndc = M.cover_nsf[M.o_cover[q]];
   double* O = M.out + M.o_elem[q];
@@ -306,89 +129,142 @@ __global__ void __launch_bounds__(128) k_mult_tc6(TCArgs M) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       int row = g + ((r & 2) ? 8 : 0), col = 8 * h + 2 * t4 + (r & 1);
-      if (row < ndr && col < ndc) O[row + ndr * col] = acc[h][r];
+      if (row < ndr && col < ndc) O[row + ndr * col] = (double)acc[h][r];
     }
 }
 
-// Three-part split, G output blocks of one row per warp (G = 2 or 4): each first-operand fragment is
-// loaded once for the blocks whose lists contain it.  Every output block takes its terms in its own
-// list order, each term rounded to FP32 once as in k_mult_tc6, so the result is the same bits for
-// every G.
-template <int kG>
-__global__ void __launch_bounds__(128) k_mult_tc6g(TCArgs M) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= M.n_groups) return;
-  const int2 grp = M.groups[w];
-  int64_t p[kG], pe[kG];
-  int nx[kG];
-  double acc[kG][2][4];
+// Two-part split (BF16x3), one output block per warp: three MMAs per pair and n8 half into FP32 accumulators, the
+// halves alternating so that neither chain waits for its own last MMA.  The next term's fragments are loaded
+// while the current term's MMAs run, and the pair after that a term earlier still, so that no load waits for
+// another.  What bounds it: the 2 KB of fragments a pair brings from L2 (32 cycles at 64 bytes per SM and cycle; it
+// takes 32 on LS.L -> LSL of the 216-atom DZP cell, 40.3 TFLOP/s; without the alternation and the early pair 38.8).
+// Not taken: groups of 2, 4 and 8 output blocks of a row that share first-operand fragments (1744, 2290 and 4118 us
+// against 1620 there: the union of their lists is longer than what they share); copies into shared memory with
+// cp.async (1732 us); 8-byte loads that skip the padding rows (2154 us: twice the requests).
+__global__ void __launch_bounds__(128) k_mult_split2(TCArgs M) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (q >= M.n_out) return;
+  const int2* pairs = M.pairs + M.ptr[q];
+  const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
+  float acc[2][4];
 #pragma unroll
-  for (int b = 0; b < kG; ++b) {
-    if (b < grp.y) { p[b] = M.ptr[grp.x + b]; pe[b] = M.ptr[grp.x + b + 1]; }
-    else { p[b] = 0; pe[b] = 0; }
-    nx[b] = p[b] < pe[b] ? M.pairs[p[b]].x : INT_MAX;
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[h][r] = 0.f;
+  struct Term { uint4 ah, al, bh, bl; };
+  auto load = [&](int2 pr) {
+    Term v;
+    v.ah = __ldg(M.xa_hi + (int64_t)pr.x * 32 + lane);
+    v.al = __ldg(M.xa_lo + (int64_t)pr.x * 32 + lane);
+    v.bh = __ldg(M.bb_hi + (int64_t)pr.y * 32 + lane);
+    v.bl = __ldg(M.bb_lo + (int64_t)pr.y * 32 + lane);
+    return v;
+  };
+  Term cur = {}, nxt = {};
+  int2 pn = make_int2(0, 0);
+  if (nt > 0) cur = load(__ldg(pairs));
+  if (nt > 1) pn = __ldg(pairs + 1);
+  for (int t = 0; t < nt; ++t) {
+    if (t + 1 < nt) nxt = load(pn);
+    if (t + 2 < nt) pn = __ldg(pairs + t + 2);
+    mma_bf16(acc[0], cur.al, cur.bh.x, cur.bh.y);
+    mma_bf16(acc[1], cur.al, cur.bh.z, cur.bh.w);
+    mma_bf16(acc[0], cur.ah, cur.bl.x, cur.bl.y);
+    mma_bf16(acc[1], cur.ah, cur.bl.z, cur.bl.w);
+    mma_bf16(acc[0], cur.ah, cur.bh.x, cur.bh.y);
+    mma_bf16(acc[1], cur.ah, cur.bh.z, cur.bh.w);
+    cur = nxt;
+  }
+  store_block(M, q, lane, acc);
+}
+
+__device__ __forceinline__ void lane_copy16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 lane_read16(uint32_t src) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+  return v;
+}
+
+// Three-part split (BF16x6): v = hi + mid + lo, one output block per warp.  Per term and n8 half the
+// six products that carry terms down to 2^-16 of hi.hi run into a zeroed FP32 accumulator, smallest
+// first (hi.lo, lo.hi, mid.mid, hi.mid, mid.hi, hi.hi), and the term's 16 x 8 result is added to FP64
+// accumulators, so the FP32 rounding spans one 16-wide contraction rather than the whole sum.  The
+// omitted products (mid.lo, lo.mid, lo.lo) and the split remainders are below 2^-23 of |a||b| per
+// element product.  The halves' MMAs alternate, as above.
+// The fragments of the next two terms are on their way to shared memory (cp.async past the L1): every lane copies
+// exactly the 16-byte pieces that it reads back, so no lane waits for another and the ring only stands in for
+// registers (62 a thread instead of 96).  What bounds it: the 3 KB a pair brings from L2 (48 cycles); it takes 61 on
+// LS.L -> LSL of the 216-atom DZP cell.  Measured on the eight products of its LNV call: three stages 12.87 ms, two
+// 13.03, four 13.95; fragments prefetched into registers 13.99, with groups of two blocks 15.5 (as above).
+constexpr int kSplitStages = 3;
+constexpr int kSplitStep = 6 * 512;                // bytes of one term: three parts of two blocks
+
+__global__ void __launch_bounds__(128) k_mult_split3(TCArgs M) {
+  __shared__ __align__(128) unsigned char smem[4][kSplitStages * kSplitStep];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = blockIdx.x * 4 + warp;
+  if (q >= M.n_out) return;
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(smem[warp]) + lane * 16;
+  const int2* pairs = M.pairs + M.ptr[q];
+  const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
+  double acc[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[h][r] = 0.0;
+  int issued = 0;
+  int2 pn = nt > 0 ? __ldg(pairs) : make_int2(0, 0), pn2 = nt > 1 ? __ldg(pairs + 1) : make_int2(0, 0);
+  auto issue = [&](int st) {
+    if (issued < nt) {
+      const uint32_t d = mine + st * kSplitStep;
+      const int64_t xo = (int64_t)pn.x * 32 + lane, bo = (int64_t)pn.y * 32 + lane;
+      lane_copy16(d, M.xa_hi + xo);
+      lane_copy16(d + 512, M.xa_mid + xo);
+      lane_copy16(d + 1024, M.xa_lo + xo);
+      lane_copy16(d + 1536, M.bb_hi + bo);
+      lane_copy16(d + 2048, M.bb_mid + bo);
+      lane_copy16(d + 2560, M.bb_lo + bo);
+      pn = pn2;
+      if (issued + 2 < nt) pn2 = __ldg(pairs + issued + 2);
+    }
+    ++issued;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k + 1 < kSplitStages; ++k) issue(k);
+  int st = 0;
+  for (int t = 0; t < nt; ++t) {
+    issue(st == 0 ? kSplitStages - 1 : st - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSplitStages - 1) : "memory");
+    const uint32_t d = mine + st * kSplitStep;
+    const uint4 ah = lane_read16(d), am = lane_read16(d + 512), al = lane_read16(d + 1024);
+    const uint4 bh = lane_read16(d + 1536), bm = lane_read16(d + 2048), bl = lane_read16(d + 2560);
+    float c[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) acc[b][h][r] = 0.0;
+      for (int r = 0; r < 4; ++r) c[h][r] = 0.f;
+    mma_bf16(c[0], ah, bl.x, bl.y);
+    mma_bf16(c[1], ah, bl.z, bl.w);
+    mma_bf16(c[0], al, bh.x, bh.y);
+    mma_bf16(c[1], al, bh.z, bh.w);
+    mma_bf16(c[0], am, bm.x, bm.y);
+    mma_bf16(c[1], am, bm.z, bm.w);
+    mma_bf16(c[0], ah, bm.x, bm.y);
+    mma_bf16(c[1], ah, bm.z, bm.w);
+    mma_bf16(c[0], am, bh.x, bh.y);
+    mma_bf16(c[1], am, bh.z, bh.w);
+    mma_bf16(c[0], ah, bh.x, bh.y);
+    mma_bf16(c[1], ah, bh.z, bh.w);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[h][r] += (double)c[h][r];
+    st = st + 1 == kSplitStages ? 0 : st + 1;
   }
-  while (true) {
-    int kc = INT_MAX;
-#pragma unroll
-    for (int b = 0; b < kG; ++b) kc = min(kc, nx[b]);
-    if (kc == INT_MAX) break;
-    const uint4 ah = __ldg(M.xa_hi + (int64_t)kc * 32 + lane);
-    const uint4 am = __ldg(M.xa_mid + (int64_t)kc * 32 + lane);
-    const uint4 al = __ldg(M.xa_lo + (int64_t)kc * 32 + lane);
-#pragma unroll
-    for (int b = 0; b < kG; ++b) {
-      if (nx[b] == kc) {
-        const int y = M.pairs[p[b]].y;
-        const uint4 bh = __ldg(M.bb_hi + (int64_t)y * 32 + lane);
-        const uint4 bm = __ldg(M.bb_mid + (int64_t)y * 32 + lane);
-        const uint4 bl = __ldg(M.bb_lo + (int64_t)y * 32 + lane);
-        float t[2][4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) t[h][r] = 0.f;
-        mma_bf16(t[0], ah, bl.x, bl.y);
-        mma_bf16(t[0], al, bh.x, bh.y);
-        mma_bf16(t[0], am, bm.x, bm.y);
-        mma_bf16(t[0], ah, bm.x, bm.y);
-        mma_bf16(t[0], am, bh.x, bh.y);
-        mma_bf16(t[0], ah, bh.x, bh.y);
-        mma_bf16(t[1], ah, bl.z, bl.w);
-        mma_bf16(t[1], al, bh.z, bh.w);
-        mma_bf16(t[1], am, bm.z, bm.w);
-        mma_bf16(t[1], ah, bm.z, bm.w);
-        mma_bf16(t[1], am, bh.z, bh.w);
-        mma_bf16(t[1], ah, bh.z, bh.w);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) acc[b][h][r] += (double)t[h][r];
-        ++p[b];
-        nx[b] = p[b] < pe[b] ? M.pairs[p[b]].x : INT_MAX;
-      }
-    }
-  }
-  const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-  for (int b = 0; b < kG; ++b) {
-    if (b < grp.y) {
-      const int q = grp.x + b;
-      const int ndr = M.prim_nsf[M.o_row[q]], ndc = M.cover_nsf[M.o_cover[q]];
-      double* O = M.out + M.o_elem[q];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          int row = g + ((r & 2) ? 8 : 0), col = 8 * h + 2 * t4 + (r & 1);
-          if (row < ndr && col < ndc) O[row + ndr * col] = acc[b][h][r];
-        }
-    }
-  }
+  store_block(M, q, lane, acc);
 }
 
 }  // namespace
@@ -414,35 +290,21 @@ static FragBuf& frag_buffer(System& S, int r, int slot, bool three = false) {
   return f;
 }
 
+// split-precision products on mma.sync, one output block per warp
 static void mat_mult_mma_sync(System& S, MixedPlan& MP, int mult_type, int ra, int rb, int rc, double* a,
-                              const double* b, double* c) {
-  int rx = mult_type == 1 ? ra : rc;
+                              const double* b, double* c, int parts) {
+  const int rx = mult_type == 1 ? ra : rc;
   const double* x = mult_type == 1 ? a : c;
   double* out = mult_type == 1 ? c : a;
-  FragBuf& fx = frag_buffer(S, rx, 0);
-  FragBuf& fb = frag_buffer(S, rb, 1);
-  to_fragments(S, rx, x, 0, 0, fx.hi.p, fx.lo.p, nullptr);
-  to_fragments(S, rb, b, 1, mult_type == 2 ? 1 : 0, fb.hi.p, fb.lo.p, nullptr);
-  launch_mult_tc(S, MP, fx.hi.p, fx.lo.p, fb.hi.p, fb.lo.p, out);
-}
-
-static void ensure_groups(System& S, MixedPlan& MP, int gi);
-static void launch_tc6_g(System& S, MixedPlan& MP, TCArgs M, int gi);
-
-// three-part split products (one output block per warp)
-static void mat_mult_split6(System& S, MixedPlan& MP, int mult_type, int ra, int rb, int rc, double* a,
-                            const double* b, double* c) {
-  int rx = mult_type == 1 ? ra : rc;
-  const double* x = mult_type == 1 ? a : c;
-  double* out = mult_type == 1 ? c : a;
-  FragBuf& fx = frag_buffer(S, rx, 0, true);
-  FragBuf& fb = frag_buffer(S, rb, 1, true);
-  to_fragments(S, rx, x, 0, 0, fx.hi.p, fx.lo.p, fx.mid.p);
-  to_fragments(S, rb, b, 1, mult_type == 2 ? 1 : 0, fb.hi.p, fb.lo.p, fb.mid.p);
+  const bool three = parts == 3;
+  FragBuf& fx = frag_buffer(S, rx, 0, three);
+  FragBuf& fb = frag_buffer(S, rb, 1, three);
+  to_fragments(S, rx, x, 0, 0, fx.hi.p, fx.lo.p, three ? fx.mid.p : nullptr);
+  to_fragments(S, rb, b, 1, mult_type == 2 ? 1 : 0, fb.hi.p, fb.lo.p, three ? fb.mid.p : nullptr);
   RangeIndex& O = *S.ranges[MP.out_range];
   if (O.nnz == 0) return;
-  ensure_groups(S, MP, 0);
   TCArgs M;
+  M.n_out = O.nnz;
   M.ptr = MP.ptr;
   M.pairs = MP.pairs;
   M.xa_hi = fx.hi.p; M.xa_lo = fx.lo.p; M.xa_mid = fx.mid.p;
@@ -450,73 +312,33 @@ static void mat_mult_split6(System& S, MixedPlan& MP, int mult_type, int ra, int
   M.o_row = O.nb_row.p; M.o_cover = O.nb_cover.p; M.o_elem = O.nb_elem.p;
   M.prim_nsf = S.dg.prim_nsf.p; M.cover_nsf = S.dg.cover_nsf.p;
   M.out = out;
-  if (MP.tuned_g6 < 0) {
-    // autotuner: groups of 1, 2 and 4 output blocks (the same bits), as for the two-part kernel
-    cudaEvent_t e0, e1;
-    CQ_CUDA(cudaEventCreate(&e0));
-    CQ_CUDA(cudaEventCreate(&e1));
-    float best[3] = {1e30f, 1e30f, 1e30f};
-    for (int gi = 0; gi < 3; ++gi) launch_tc6_g(S, MP, M, gi);
-    for (int round = 0; round < 3; ++round)
-      for (int gi = 0; gi < 3; ++gi) {
-        CQ_CUDA(cudaEventRecord(e0, S.stream));
-        launch_tc6_g(S, MP, M, gi);
-        CQ_CUDA(cudaEventRecord(e1, S.stream));
-        CQ_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CQ_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        best[gi] = std::min(best[gi], ms);
-      }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    int pick = 0;
-    for (int gi = 1; gi < 3; ++gi)
-      if (best[gi] < 0.95f * best[pick]) pick = gi;
-    for (int gi = 0; gi < 3; ++gi) MP.tune_ms6[gi] = best[gi];
-    MP.tuned_g6 = pick;
-  }
-  const int forced = S.split_group == 1 ? 0 : S.split_group == 2 ? 1 : S.split_group == 4 ? 2 : -1;
-  launch_tc6_g(S, MP, M, forced >= 0 ? forced : MP.tuned_g6);
-}
-
-// gi = 0: one output block per warp with prefetch; 1, 2: groups of 2 and 4 blocks of one row
-static void launch_tc6_g(System& S, MixedPlan& MP, TCArgs M, int gi) {
-  static const int kGi[3] = {0, 1, 2};   // index into the group sizes 1, 2, 4, 8
-  ensure_groups(S, MP, kGi[gi]);
-  M.groups = MP.groups[kGi[gi]].p;
-  M.n_groups = MP.n_groups[kGi[gi]];
-  if (M.n_groups == 0) return;
-  const int grid = (M.n_groups * 32 + 127) / 128;
-  if (gi == 0) k_mult_tc6<<<grid, 128, 0, S.stream>>>(M);
-  else if (gi == 1) k_mult_tc6g<2><<<grid, 128, 0, S.stream>>>(M);
-  else k_mult_tc6g<4><<<grid, 128, 0, S.stream>>>(M);
+  const int grid = (int)(((int64_t)M.n_out * 32 + 127) / 128);
+  if (three) k_mult_split3<<<grid, 128, 0, S.stream>>>(M);
+  else k_mult_split2<<<grid, 128, 0, S.stream>>>(M);
   S.launches++;
   CQ_CUDA(cudaGetLastError());
 }
 
-// Kernel choice of a split-precision product: the system's setting, or (setting -1) a fixed rule on
-// the product's tile plan, so that a product always runs the same kernel (and gives the same bits)
-// whatever else runs on the device: the tcgen05 tiles where at least kTileMinFill of their issued
-// tensor work is useful (3 x the product's flops / issued flops), else the per-block mma.sync kernel.
-// Measured on B200 (4096-atom DZP cell, the nine products of an LNV call): the tiles issue 330-850
-// TFLOP/s at useful fractions of 0.056-0.114 and the per-block kernel reaches 25-31 TFLOP/s useful;
-// the tiles were faster for the product with fraction 0.114 (31.1 against 29.3) and slower below.
+// Kernel choice of a two-part split product: the system's setting, or (setting -1) a fixed rule, so that a product
+// always runs the same kernel (and gives the same bits) whatever else runs on the device: the tcgen05 tiles where
+// the product has at least kTileMinBlocks output blocks and at least kTileMinFill of the tiles' tensor work is useful,
+// else the per-block mma.sync kernel.  Measured on LS.L -> LSL of DZP cells (useful fraction 0.114; blocks / tiles,
+// TFLOP/s): 216 atoms, 0.50 M output blocks, 40.3 / 28.9; 512 atoms, 1.18 M, 37.5 / 30.6; 1728 atoms, 3.99 M, 30.5 /
+// 34.1 (its fragments have outgrown the L2); 4096 atoms 29.3 / 31.1.  On products with fractions of 0.056 to 0.10
+// the blocks were faster at every size.  Below the block count no tile plan is built.
+constexpr int kTileMinBlocks = 2500000;
 constexpr double kTileMinFill = 0.11;
 
 void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a, const double* b, double* c,
                     int parts) {
   MixedPlan& MP = get_mixed_plan(S, mult_type, ra, rb, rc);
-  if (parts == 3) {
-    mat_mult_split6(S, MP, mult_type, ra, rb, rc, a, b, c);
-    return;
-  }
-  const bool tiles_ok = umma_usable(S, mult_type, ra, rb, rc);
   int k = S.mixed_kernel;
-  if (k == 0 && !tiles_ok) k = 1;
+  if (parts == 3) k = 1;
+  if (k == 0 && !umma_usable(S, mult_type, ra, rb, rc)) k = 1;
   if (k < 0) {
     if (MP.kernel < 0) {
       MP.kernel = 1;
-      if (tiles_ok) {
+      if (S.ranges[MP.out_range]->nnz >= kTileMinBlocks && umma_usable(S, mult_type, ra, rb, rc)) {
         const UmmaPlan& U = get_umma_plan(S, mult_type, ra, rb, rc);
         if (U.issued_flops > 0 && 3.0 * (double)U.flops / (double)U.issued_flops >= kTileMinFill) MP.kernel = 0;
       }
@@ -524,79 +346,7 @@ void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a,
     k = MP.kernel;
   }
   if (k == 0) mat_mult_umma(S, mult_type, ra, rb, rc, a, b, c);
-  else mat_mult_mma_sync(S, MP, mult_type, ra, rb, rc, a, b, c);
-}
-
-static void ensure_groups(System& S, MixedPlan& MP, int gi) {
-  static const int kGs[4] = {1, 2, 4, 8};
-  if (MP.n_groups[gi] < 0) {
-    // groups of up to G consecutive output blocks of one row
-    RangeIndex& O = *S.ranges[MP.out_range];
-    const int G = kGs[gi];
-    std::vector<int2> grp;
-    for (int p = 0; p < S.geo.n_prim; ++p)
-      for (int s0 = O.h_row_ptr[p]; s0 < O.h_row_ptr[p + 1]; s0 += G)
-        grp.push_back(make_int2(s0, std::min(G, O.h_row_ptr[p + 1] - s0)));
-    MP.n_groups[gi] = (int)grp.size();
-    MP.groups[gi].upload(grp, S.stream);
-  }
-}
-
-static void launch_tc_g(System& S, MixedPlan& MP, TCArgs M, int gi) {
-  ensure_groups(S, MP, gi);
-  M.groups = MP.groups[gi].p;
-  M.n_groups = MP.n_groups[gi];
-  if (M.n_groups == 0) return;
-  const int grid = (M.n_groups * 32 + 127) / 128;
-  if (gi == 0) k_mult_tc1<<<grid, 128, 0, S.stream>>>(M);
-  else if (gi == 1) k_mult_tc<2><<<grid, 128, 0, S.stream>>>(M);
-  else if (gi == 2) k_mult_tc<4><<<grid, 128, 0, S.stream>>>(M);
-  else k_mult_tc<8><<<grid, 128, 0, S.stream>>>(M);
-  S.launches++;
-  CQ_CUDA(cudaGetLastError());
-}
-
-void launch_mult_tc(System& S, MixedPlan& MP, const uint4* xa_hi, const uint4* xa_lo, const uint4* bb_hi,
-                    const uint4* bb_lo, double* out) {
-  RangeIndex& O = *S.ranges[MP.out_range];
-  TCArgs M;
-  M.ptr = MP.ptr;
-  M.pairs = MP.pairs;
-  M.xa_hi = xa_hi; M.xa_lo = xa_lo; M.bb_hi = bb_hi; M.bb_lo = bb_lo;
-  M.xa_mid = nullptr; M.bb_mid = nullptr;
-  M.o_row = O.nb_row.p; M.o_cover = O.nb_cover.p; M.o_elem = O.nb_elem.p;
-  M.prim_nsf = S.dg.prim_nsf.p; M.cover_nsf = S.dg.cover_nsf.p;
-  M.out = out;
-  if (O.nnz == 0) return;
-  if (MP.tuned_g < 0) {
-    // autotuner: each group size once warm, then three interleaved timed rounds; the fastest
-    // round counts, and a smaller group replaces a larger one only when it is 5 % faster.  Every launch overwrites
-    // the whole output with the same values.
-    cudaEvent_t e0, e1;
-    CQ_CUDA(cudaEventCreate(&e0));
-    CQ_CUDA(cudaEventCreate(&e1));
-    float best[4] = {1e30f, 1e30f, 1e30f, 1e30f};
-    for (int gi = 0; gi < 4; ++gi) launch_tc_g(S, MP, M, gi);
-    for (int round = 0; round < 3; ++round)
-      for (int gi = 0; gi < 4; ++gi) {
-        CQ_CUDA(cudaEventRecord(e0, S.stream));
-        launch_tc_g(S, MP, M, gi);
-        CQ_CUDA(cudaEventRecord(e1, S.stream));
-        CQ_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CQ_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        best[gi] = std::min(best[gi], ms);
-      }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    int pick = 3;
-    for (int gi = 0; gi < 3; ++gi)
-      if (best[gi] < 0.95f * best[pick]) pick = gi;
-    for (int gi = 0; gi < 4; ++gi) MP.tune_ms[gi] = best[gi];
-    MP.tuned_g = pick;
-  }
-  const int forced = S.split_group == 1 ? 0 : S.split_group == 2 ? 1 : S.split_group == 4 ? 2 : S.split_group == 8 ? 3 : -1;
-  launch_tc_g(S, MP, M, forced >= 0 ? forced : MP.tuned_g);
+  else mat_mult_mma_sync(S, MP, mult_type, ra, rb, rc, a, b, c, parts);
 }
 
 }  // namespace cqb

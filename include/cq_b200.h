@@ -184,8 +184,8 @@ int cq_product_work(cq_system* sys, int mult_type, int ra, int rb, int rc, int64
 
 /* Kernel record of one product: the FP64 kernel variant chosen for it (-1 before the product's
  * first call with the automatic choice) and the timed milliseconds of each variant (ms[7], 0 = not
- * timed; the FP64 choice is a rule and times none); for its split-precision form the output blocks per warp it chose (1, 2, 4 or 8; -1 =
- * not tuned yet) and the timed milliseconds of those four group sizes (group_ms[4]). */
+ * timed; the FP64 choice is a rule and times none); for its split-precision form the output blocks per
+ * warp (1; -1 = has not run yet) and the timed milliseconds of four group sizes (group_ms[4], 0). */
 int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int* variant, float* ms, int* group,
                       float* group_ms);
 
@@ -287,8 +287,8 @@ int cq_generate_SH(cq_system* sys, int r, int which, uint64_t seed, double* out)
 #define CQ_OPT_BLOCKING_SYNC 2
 /* CQ_OPT_MIXED_KERNEL: kernel of the CQ_PREC_BF16X3 products (CQ_PREC_BF16X6 products always run on
  * mma.sync: the tcgen05 tiles accumulate a whole contraction in FP32).  -1 (default) = chosen per product
- * by a fixed rule (the tiles where at least 11 % of their issued tensor work is useful), so a product
- * always gives the same bits; 0 = dense 128 x 128 tiles on the tcgen05 tensor cores with TMEM
+ * by a fixed rule (the tiles where at least 11 % of their issued tensor work is useful, from 2.5 million
+ * output blocks on), so a product always gives the same bits; 0 = dense 128 x 128 tiles on the tcgen05 tensor cores with TMEM
  * accumulators, operands staged by bulk copies (every block size 4..16; other systems use 1);
  * 1 = one padded 16 x 16 block per warp-level mma.sync. */
 #define CQ_OPT_MIXED_KERNEL 3
@@ -297,9 +297,9 @@ int cq_generate_SH(cq_system* sys, int r, int which, uint64_t seed, double* out)
  * synchronises (cq_mat_mult_host, cq_synchronize, the chain's waits) returns CQ_ERR_TIMEOUT; the
  * context stays usable and the product's output is not valid.  One product, then back to 0. */
 #define CQ_OPT_TEST_STALL 4
-/* CQ_OPT_SPLIT_GROUP: output blocks per warp of the mma.sync split-precision kernels.  -1 (default)
- * = chosen per product by the autotuner; 1, 2, 4 (and 8, two-part split only) = that group size.
- * Every group size gives the same bits (each output block sums its own terms in its own order). */
+/* CQ_OPT_SPLIT_GROUP: output blocks per warp of the mma.sync split-precision kernels, -1, 1, 2, 4 or 8.
+ * Accepted for existing callers and without effect: every group size gave the same bits, and one block
+ * per warp, the fastest on every product measured, is what all of them run. */
 #define CQ_OPT_SPLIT_GROUP 5
 int cq_system_set_option(cq_system* sys, int option, int value);
 
