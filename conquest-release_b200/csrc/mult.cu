@@ -935,21 +935,29 @@ __global__ void __launch_bounds__(64) k_mult_dmma(MultArgs M, const int* __restr
   const int2* pairs = M.pairs + M.ptr[q];
   const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
   const uint32_t w0 = smem_addr(W);
-  int2 pn = gp < nt ? __ldcs(pairs + gp) : make_int2(-1, -1);      // the group's pair, loaded a round ahead
-  for (int t0 = 0; t0 < nt; t0 += 4) {
-    const int2 pr = pn;
-    pn = t0 + 4 + gp < nt ? __ldcs(pairs + t0 + 4 + gp) : make_int2(-1, -1);
-    int nk = 0;
-    bool px = false, pb = false;                  // 8-byte phases of the copies
+  // the group's pair of the next round with its addresses looked up, and the pair of the round after that
+  struct Term { const double *x, *b; int nk; };
+  auto look_up = [&](int2 pr) {
+    Term v = {nullptr, nullptr, 0};
     if (pr.x >= 0) {
-      const double* Xg = M.x + (U > 0 ? (int64_t)pr.x * (U * U) : M.x_elem[pr.x]);
-      const double* Bg = M.b + (U > 0 ? (int64_t)pr.y * (U * U) : M.b_elem[pr.y]);
-      nk = U > 0 ? U : (TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]]);
-      px = ((uintptr_t)Xg >> 3) & 1;
-      pb = ((uintptr_t)Bg >> 3) & 1;
-      group_copy<U, 8>(w0 + gp * kStride, Xg, ndi * nk, l);
-      group_copy<U, 8>(w0 + (4 + gp) * kStride, Bg, nk * ndo, l);
+      v.x = M.x + (U > 0 ? (int64_t)pr.x * (U * U) : M.x_elem[pr.x]);
+      v.b = M.b + (U > 0 ? (int64_t)pr.y * (U * U) : M.b_elem[pr.y]);
+      v.nk = U > 0 ? U : (TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]]);
     }
+    return v;
+  };
+  auto pair_of = [&](int k) { return k < nt ? __ldcs(pairs + k) : make_int2(-1, -1); };
+  Term next = look_up(pair_of(gp));
+  int2 pn = pair_of(4 + gp);
+  for (int t0 = 0; t0 < nt; t0 += 4) {
+    const int nk = next.nk;                       // 0 past the list's end
+    const bool px = ((uintptr_t)next.x >> 3) & 1, pb = ((uintptr_t)next.b >> 3) & 1;   // 8-byte phases of the copies
+    if (nk > 0) {
+      group_copy<U, 8>(w0 + gp * kStride, next.x, ndi * nk, l);
+      group_copy<U, 8>(w0 + (4 + gp) * kStride, next.b, nk * ndo, l);
+    }
+    next = look_up(pn);
+    pn = pair_of(t0 + 8 + gp);
     cp_async_commit();
     const unsigned mx = __ballot_sync(kFull, px), mb = __ballot_sync(kFull, pb);
     // contraction offsets of the pairs
@@ -1379,9 +1387,11 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
     const int grid = (M.n_out + 1) / 2;
     if (P.mult_type == 1) {
       if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
+      else if (S.max_nsf <= 13) k_mult_dmma<1, 0, 13><<<grid, 64, 0, st>>>(M, P.order.p);
       else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
     } else {
       if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
+      else if (S.max_nsf <= 13) k_mult_dmma<2, 0, 13><<<grid, 64, 0, st>>>(M, P.order.p);
       else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
     }
     S.launches++;
