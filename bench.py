@@ -376,7 +376,7 @@ def main():
                          "call on the 512-atom SZ, 216-atom DZP and 4096-atom DZP cells); forms216: one 216-atom "
                          "DZP solve in each precision form")
     ap.add_argument("--precision", default="fp64", choices=["fp64", "fma", "bf16x3", "bf16x6", "fp64tc"])
-    ap.add_argument("--variant", type=int, default=None, help="FP64 4x4 product kernel variant (-1 autotuned, 0..3, 5, 6)")
+    ap.add_argument("--variant", type=int, default=None, help="FP64 4x4 product kernel variant (-1 chosen by size, 0..6)")
     ap.add_argument("--mixed-kernel", type=int, default=-1, choices=[-1, 0, 1],
                     help="split-precision products: -1 = chosen per product by the tile plan's useful fraction "
                          "(default), 0 = tcgen05 tiles, 1 = one block per mma.sync warp")
@@ -556,7 +556,7 @@ def main():
             "parity": fixture_parity(res),
             "mixed_vs_fp64": mixed,
             "block_mult_tflops": (prof["flops"] / (prof["ms"] / 1e3) / 1e12) if prof["ms"] > 0 else None,
-            "roofline": {"bound": "hbm", "kernel": "FP64 4x4 block products (autotuned k_mult_nd4_warp / k_mult_nd4_quad)", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "FP64 4x4 block products (k_mult_nd4_warp / _row / _quad, chosen by size)", "achieved": achieved,
                          "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic[0], "traffic_launch": traffic[1],
                          "traffic_launch_algorithmic_bytes": traffic[2], "launches": prof["launches"],

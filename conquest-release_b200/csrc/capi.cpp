@@ -413,7 +413,7 @@ int cq_system_set_option(cq_system* sys, int option, int value) {
   return guarded([&] {
     check_sys(sys);
     if (option == CQ_OPT_MULT_VARIANT) {
-      CQ_CHECK(value >= -1 && value <= 6, CQ_ERR_ARG, "mult variant must be -1 (autotuned) or 0..6");
+      CQ_CHECK(value >= -1 && value <= 6, CQ_ERR_ARG, "mult variant must be -1 (chosen by size) or 0..6");
       sys->S.mult_variant = value;
     } else if (option == CQ_OPT_BLOCKING_SYNC) {
       sys->S.blocking_sync = value != 0;
@@ -425,7 +425,7 @@ int cq_system_set_option(cq_system* sys, int option, int value) {
       sys->S.mixed_kernel = value;
     } else if (option == CQ_OPT_SPLIT_GROUP) {
       CQ_CHECK(value == -1 || value == 1 || value == 2 || value == 4 || value == 8, CQ_ERR_ARG,
-               "split group must be -1 (autotuned), 1, 2, 4 or 8");
+               "split group must be -1, 1, 2, 4 or 8");
       // accepted as before; every product takes one output block per warp, the fastest size on all of them
     } else {
       throw Error(CQ_ERR_ARG, "unknown option");
