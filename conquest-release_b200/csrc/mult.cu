@@ -54,6 +54,9 @@ struct MultArgs {
   double* __restrict__ out;
 };
 
+// Output block at a slot of the launch: the plan's order where it has been built, else the stored order.
+__device__ __forceinline__ int ordered(const int* __restrict__ order, int slot) { return order ? order[slot] : slot; }
+
 // Generic block sizes (nd <= 16): one warp per output block, up to 8 elements per lane.
 template <int TYPE, bool EXACT>
 __global__ void __launch_bounds__(256) k_mult_generic(MultArgs M) {
@@ -315,7 +318,7 @@ __device__ __forceinline__ void warp_nd4_staged(const MultArgs& M, const int* __
   const int lane = threadIdx.x & 31;
   const int slot = base + lane;
   const bool has = slot < M.n_out;
-  const int q = has ? order[slot] : 0;
+  const int q = has ? ordered(order, slot) : 0;
   const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
   const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
   const int steps = __reduce_max_sync(kFull, nt);
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(128, 2) k_mult_nd4_bulk(MultArgs M, const int*
   if (base >= M.n_out) return;                  // whole warp (nothing waits on its barriers)
   const int slot = base + lane;
   const bool has = slot < M.n_out;
-  const int q = has ? order[slot] : 0;
+  const int q = has ? ordered(order, slot) : 0;
   const int64_t t = has ? M.ptr[q] : 0;
   const int64_t tend = has ? M.ptr[q + 1] : 0;
   double acc[16];
@@ -606,7 +609,7 @@ __global__ void __launch_bounds__(128) k_mult_nd4_quad(MultArgs M, const int* __
   if (base >= M.n_out) return;                   // whole warp
   const int slot = base + qd;
   const bool has = slot < M.n_out;
-  const int q = has ? order[slot] : 0;
+  const int q = has ? ordered(order, slot) : 0;
   const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
   const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
   const int steps = __reduce_max_sync(kFull, nt);
@@ -780,7 +783,7 @@ __device__ __forceinline__ void warp_group_rows(const MultArgs& M, const int* __
   const unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31, g = lane / LPB, l = lane % LPB;
   const bool has = base + g < M.n_out;
-  const int q = has ? order[base + g] : 0;
+  const int q = has ? ordered(order, base + g) : 0;
   const int ndi = FULL ? R : M.prim_nsf[M.o_row[q]];
   const int ndo = U > 0 ? U : M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
   int c[H];
@@ -873,7 +876,7 @@ __device__ __forceinline__ void warp_group(const MultArgs& M, const int* __restr
     // several sizes: a warp whose blocks all have four rows, or all MAXND, runs a tile of exactly that height
     // (the order keeps blocks of one row count together)
     const int s = min(base + (threadIdx.x & 31) / LPB, M.n_out - 1);
-    const int ndi = M.prim_nsf[M.o_row[order[s]]];
+    const int ndi = M.prim_nsf[M.o_row[ordered(order, s)]];
     if (__all_sync(0xffffffffu, ndi == 4)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, 4, true>(M, order, base, W);
     else if (__all_sync(0xffffffffu, ndi == MAXND)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, true>(M, order, base, W);
     else warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, false>(M, order, base, W);
@@ -919,7 +922,7 @@ __global__ void __launch_bounds__(64) k_mult_dmma(MultArgs M, const int* __restr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = blockIdx.x * 2 + warp;
   if (slot >= M.n_out) return;                    // whole warp
-  const int q = order[slot];
+  const int q = ordered(order, slot);
   const int g = lane >> 2, t = lane & 3;          // fragment row / column and contraction index
   const int gp = lane >> 3, l = lane & 7;         // staging: pair and lane of its group
   unsigned char* W = smem[warp];
@@ -1159,9 +1162,17 @@ __global__ void __launch_bounds__(256) k_order_fill(OrderKey key, int n, int bin
 }
 }  // namespace
 
-static void ensure_order(System& S, ProductPlan& P) {
+static bool capturing(const System& S) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  CQ_CUDA(cudaStreamIsCapturing(S.stream, &status));
+  return status != cudaStreamCaptureStatusNone;
+}
+
+// The plan's output order, built on its first use, which allocates and waits for the stream: a launch that is being
+// captured into a graph before then runs in the stored order instead (null: the same results).
+static const int* output_order(System& S, ProductPlan& P) {
   const RangeIndex& O = *S.ranges[P.out_range];
-  if (P.order.n != 0 || O.nnz == 0) return;
+  if (P.order.n != 0 || O.nnz == 0 || capturing(S)) return P.order.p;
   OrderKey key;
   key.ptr = P.ptr.p;
   key.o_row = O.nb_row.p;
@@ -1182,6 +1193,7 @@ static void ensure_order(System& S, ProductPlan& P) {
   k_order_fill<<<tiles, 256, bins * sizeof(int), S.stream>>>(key, O.nnz, bins, first.p, P.order.p);
   S.launches += 2;
   CQ_CUDA(cudaGetLastError());
+  return P.order.p;
 }
 
 // Dynamic shared memory above 48 KB has to be allowed per kernel (once per system and kernel).
@@ -1200,14 +1212,16 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   const int T = 256;
   RangeIndex& O = P.mult_type == 1 ? *S.ranges[P.rc] : *S.ranges[P.ra];
   RangeIndex& X = P.mult_type == 1 ? *S.ranges[P.ra] : *S.ranges[P.rc];
-  if (nd4 && (variant >= 3)) ensure_order(S, P);
+  // the row kernel's tiles are uploaded on its first use: a launch captured before then takes the warp-staged kernel
+  if (nd4 && variant == 4 && P.mult_type == 2 && P.n_row_tiles < 0 && capturing(S)) variant = 3;
+  const int* order = nd4 && variant >= 3 ? output_order(S, P) : nullptr;
   if (nd4 && variant == 6) {
     const int grid = (M.n_out + 127) / 128;
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
     int* err = device_timeout_word(S);
     auto launch = [&](auto kern) {
       allow_smem(S, kern, (int)smem);
-      kern<<<grid, 128, smem, st>>>(M, P.order.p, err);
+      kern<<<grid, 128, smem, st>>>(M, order, err);
     };
     if (P.mult_type == 1) {
       if (exact) launch(k_mult_nd4_bulk<1, true>); else launch(k_mult_nd4_bulk<1, false>);
@@ -1217,11 +1231,11 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   } else if (nd4 && variant == 5) {
     const int grid = (M.n_out + 31) / 32;        // 8 output blocks per warp, 4 warps per CTA
     if (P.mult_type == 1) {
-      if (exact) k_mult_nd4_quad<1, true, 4><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_quad<1, false, 4><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_quad<1, true, 4><<<grid, 128, 0, st>>>(M, order);
+      else k_mult_nd4_quad<1, false, 4><<<grid, 128, 0, st>>>(M, order);
     } else {
-      if (exact) k_mult_nd4_quad<2, true, 4><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_quad<2, false, 4><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_quad<2, true, 4><<<grid, 128, 0, st>>>(M, order);
+      else k_mult_nd4_quad<2, false, 4><<<grid, 128, 0, st>>>(M, order);
     }
   } else if (nd4 && variant == 4 && P.mult_type == 2) {
     if (P.n_row_tiles < 0) {
@@ -1241,11 +1255,11 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   } else if (nd4 && (variant == 3 || variant == 4)) {
     const int grid = (M.n_out + 127) / 128;
     if (P.mult_type == 1) {
-      if (exact) k_mult_nd4_warp<1, true><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_warp<1, false><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_warp<1, true><<<grid, 128, 0, st>>>(M, order);
+      else k_mult_nd4_warp<1, false><<<grid, 128, 0, st>>>(M, order);
     } else {
-      if (exact) k_mult_nd4_warp<2, true><<<grid, 128, 0, st>>>(M, P.order.p);
-      else k_mult_nd4_warp<2, false><<<grid, 128, 0, st>>>(M, P.order.p);
+      if (exact) k_mult_nd4_warp<2, true><<<grid, 128, 0, st>>>(M, order);
+      else k_mult_nd4_warp<2, false><<<grid, 128, 0, st>>>(M, order);
     }
   } else if (nd4 && variant == 2) {
     constexpr int kChunk = 256;                 // 32 KiB of operand blocks per chunk
@@ -1281,10 +1295,10 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) k_mult_nd4<2, true><<<grid, T, 0, st>>>(M); else k_mult_nd4<2, false><<<grid, T, 0, st>>>(M);
     }
   } else if (variant == 4) {
-    ensure_order(S, P);
+    order = output_order(S, P);
     auto launch = [&](auto kern, int blocks, int warp_bytes) {
       allow_smem(S, kern, 2 * warp_bytes);
-      kern<<<(M.n_out + 2 * blocks - 1) / (2 * blocks), 64, 2 * warp_bytes, st>>>(M, P.order.p);
+      kern<<<(M.n_out + 2 * blocks - 1) / (2 * blocks), 64, 2 * warp_bytes, st>>>(M, order);
     };
     auto by_size = [&](auto type, auto ex) {
       constexpr int TY = decltype(type)::value;
@@ -1383,16 +1397,16 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   // those of the CUDA-core kernels (checked on B200), about three times faster on 13 x 13 blocks
   // (unless a CUDA-core variant is forced with CQ_OPT_MULT_VARIANT)
   if (exact == kPrecFp64Tensor || (exact == 0 && S.max_nsf > 8 && S.mult_variant == kVariantAuto)) {
-    ensure_order(S, P);
+    const int* order = output_order(S, P);
     const int grid = (M.n_out + 1) / 2;
     if (P.mult_type == 1) {
-      if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
-      else if (S.max_nsf <= 13) k_mult_dmma<1, 0, 13><<<grid, 64, 0, st>>>(M, P.order.p);
-      else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
+      if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, order);
+      else if (S.max_nsf <= 13) k_mult_dmma<1, 0, 13><<<grid, 64, 0, st>>>(M, order);
+      else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, order);
     } else {
-      if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, P.order.p);
-      else if (S.max_nsf <= 13) k_mult_dmma<2, 0, 13><<<grid, 64, 0, st>>>(M, P.order.p);
-      else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, P.order.p);
+      if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, order);
+      else if (S.max_nsf <= 13) k_mult_dmma<2, 0, 13><<<grid, 64, 0, st>>>(M, order);
+      else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, order);
     }
     S.launches++;
     CQ_CUDA(cudaGetLastError());
@@ -1410,7 +1424,7 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   }
 }
 
-void ensure_product_order(System& S, ProductPlan& P) { ensure_order(S, P); }
+void ensure_product_order(System& S, ProductPlan& P) { output_order(S, P); }
 
 // Products of independent systems (or of one system) in persistent launches on `st` (up to kBatchMax
 // products each).  The caller orders `st` after the work the operands depend on and the systems' later
@@ -1439,8 +1453,7 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
     BatchProduct bp;
     bp.M = product_args(S, P, it.a, it.b, it.c, &nd4);
     if (bp.M.n_out == 0) continue;
-    CQ_CHECK(P.order.p != nullptr, CQ_ERR_STATE, "batched product without its output order (ensure_product_order)");
-    bp.order = P.order.p;
+    bp.order = P.order.p;              // built by ensure_product_order on the system's stream; null under capture
     bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) |
               (nd4 ? kBatchNd4 : S.uniform_nsf == 13 ? kBatchU13 : S.max_nsf <= 13 ? kBatchMax13 : kBatchMax16);
     if (B.n_prod == kBatchMax) { flush(); B.unit_off[0] = 0; }
