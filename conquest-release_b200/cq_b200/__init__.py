@@ -319,8 +319,8 @@ class System:
         check(lib().cq_system_set_option(self._h, 5, int(g)))
 
     def set_mixed_kernel(self, k):
-        """Kernel of the split-precision products: -1 = chosen per product by the tile plan's useful fraction
-        (default), 0 = tcgen05 tiles, 1 = one block per mma.sync warp."""
+        """Kernel of the two-part split products: -1 = chosen per product by split_kernel_rule (default),
+        0 = tcgen05 tiles, 1 = one block per mma.sync warp."""
         check(lib().cq_system_set_option(self._h, 3, int(k)))
 
     def matrix_sum(self, ra, a, alpha, rb, b, beta):
@@ -574,6 +574,14 @@ def solve_cubic(a, b, c, guess):
     x = c_double()
     check(lib().cq_solve_cubic(c_double(a), c_double(b), c_double(c), c_double(guess), ctypes.byref(x)))
     return x.value
+
+
+def split_kernel_rule(n_pairs, flops, issued_flops, b_blocks):
+    """Kernel a two-part split product of these counts runs: 0 = tcgen05 tiles, 1 = one block per mma.sync warp."""
+    k = c_int()
+    check(lib().cq_split_kernel_rule(c_int64(int(n_pairs)), c_int64(int(flops)), c_double(issued_flops),
+                                     c_int64(int(b_blocks)), ctypes.byref(k)))
+    return k.value
 
 
 def pulay_alphas(ipulay, Aij, n, max_n):

@@ -340,6 +340,13 @@ int cq_product_tensor_work(cq_system* sys, int mult_type, int ra, int rb, int rc
   });
 }
 
+int cq_split_kernel_rule(int64_t n_pairs, int64_t flops, double issued_flops, int64_t b_blocks, int* kernel) {
+  return guarded([&] {
+    CQ_CHECK(kernel && n_pairs >= 0 && flops >= 0 && b_blocks >= 0, CQ_ERR_ARG, "bad argument");
+    *kernel = split_tiles_pay(n_pairs, flops, issued_flops, b_blocks) ? 0 : 1;
+  });
+}
+
 int cq_matrix_sum(cq_system* sys, int ra, double* a_dev, double alpha, int rb, const double* b_dev, double beta) {
   return guarded([&] {
     check_sys(sys); check_range(sys, ra); check_range(sys, rb);

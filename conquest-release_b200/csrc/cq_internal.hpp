@@ -293,7 +293,7 @@ struct System {
   std::map<std::pair<int, int>, FragBuf> frags;   // (range, slot) fragment buffers of the mixed products
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<UmmaPlan>> uplans;   // tensor-core tile plans
   int mixed_kernel = -1;          // split-precision products: 0 = tcgen05 tiles (umma.cu), 1 = mma.sync per block,
-                                  // -1 = chosen per product by the tile plan's useful fraction
+                                  // -1 = chosen per product (split_tiles_pay)
   int* umma_err_host = nullptr;   // mapped host word set by a tensor-core product whose bounded wait ran out
   int umma_test_stall = 0;        // test hook (CQ_OPT_TEST_STALL): the next tensor-core product stalls
   int* umma_err_dev = nullptr;
@@ -364,13 +364,15 @@ void to_fragments(System& S, int r, const double* src, int role_b, int trans, ui
 // `exact` argument of launch_mat_mult: 1 = the reference kernel's separate multiply and add, 0 = fused
 // multiply-add, kPrecFp64Tensor = FP64 on the tensor cores (DMMA); the values of CQ_PREC_* in the C ABI
 constexpr int kPrecFp64Tensor = 4;
-// parts = 2: BF16x3 (tcgen05 tiles or mma.sync blocks by the fill rule); parts = 3: BF16x6 (mma.sync)
+// parts = 2: BF16x3 (tcgen05 tiles or mma.sync blocks by split_tiles_pay); parts = 3: BF16x6 (mma.sync)
+bool split_tiles_pay(int64_t n_pairs, int64_t flops, double issued_flops, int64_t b_blocks);
 void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a, const double* b, double* c,
                     int parts = 2);
 
 // umma.cu
 UmmaPlan& get_umma_plan(System& S, int mult_type, int ra, int rb, int rc);
-bool umma_usable(System& S, int mult_type, int ra, int rb, int rc);
+bool umma_usable(const System& S);   // every block size in 4..16
+double umma_issued_estimate(System& S, int mult_type, int ra, int rb, int rc);   // UmmaPlan::issued_flops from a sample
 void mat_mult_umma(System& S, int mult_type, int ra, int rb, int rc, double* a, const double* b, double* c);
 void umma_check(System& S);       // throws CQ_ERR_TIMEOUT if a kernel's bounded wait ran out
 int* device_timeout_word(System& S);   // mapped host word the bounded waits of the system's kernels set

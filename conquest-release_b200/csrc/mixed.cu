@@ -319,29 +319,39 @@ static void mat_mult_mma_sync(System& S, MixedPlan& MP, int mult_type, int ra, i
   CQ_CUDA(cudaGetLastError());
 }
 
-// Kernel choice of a two-part split product: the system's setting, or (setting -1) a fixed rule, so that a product
-// always runs the same kernel (and gives the same bits) whatever else runs on the device: the tcgen05 tiles where
-// the product has at least kTileMinBlocks output blocks and at least kTileMinFill of the tiles' tensor work is useful,
-// else the per-block mma.sync kernel.  Measured on LS.L -> LSL of DZP cells (useful fraction 0.114; blocks / tiles,
-// TFLOP/s): 216 atoms, 0.50 M output blocks, 40.3 / 28.9; 512 atoms, 1.18 M, 37.5 / 30.6; 1728 atoms, 3.99 M, 30.5 /
-// 34.1 (its fragments have outgrown the L2); 4096 atoms 29.3 / 31.1.  On products with fractions of 0.056 to 0.10
-// the blocks were faster at every size.  Below the block count no tile plan is built.
-constexpr int kTileMinBlocks = 2500000;
+// Kernel choice of a two-part split product: the system's setting, or (setting -1) a fixed rule on the product's counts,
+// so that a product always runs the same kernel (and gives the same bits) whatever else runs on the device.  Two costs
+// are compared:
+//  - a block per mma.sync warp: 18 us and a time per pair, which is that of the 2 KB of fragments it fetches: 105 to
+//    118 ps with B's fragments (1 KB per block) well inside the L2, 140 to 151 ps where they are as large as it;
+//  - tcgen05 tiles: 40 us and the tensor work they issue, at 690 to 890 TFLOP/s once there are a few hundred tiles.
+// The tiles are taken only where at least kTileMinFill of that work is useful: the bound that this choice has always had
+// (dense products of 4 x 4 blocks lie under it and would gain: 2288 / 208 on a 300-atom cluster).  Measured in us, blocks / tiles: LS.L -> LSL of DZP cells (26, 16 -> 42
+// bohr) 216 atoms 1549 / 2162, 512 atoms 4004 / 4897, 1000 atoms 9267 / 8615, 1728 atoms 16655 / 14643; 20, 20 -> 40 bohr
+// 512 atoms 5439 / 5040, 1000 atoms 10891 / 8941; 300-atom clusters (16, 16) 236 / 270, (20, 20) 594 / 499, (32, 32)
+// 2387 / 1252, and of 4- and 13-orbital atoms 2318 / 470; 100 atoms (16, 16) 55 / 66, (20, 20) 91 / 79.
 constexpr double kTileMinFill = 0.11;
+constexpr int64_t kTileMinPairs = 300000;     // fewer never pay: no estimate of the tiles' work is made
+
+bool split_tiles_pay(int64_t n_pairs, int64_t flops, double issued_flops, int64_t b_blocks) {
+  if (n_pairs < kTileMinPairs || issued_flops <= 0.0 || 3.0 * (double)flops < kTileMinFill * issued_flops) return false;
+  const double mb = (double)b_blocks * 1024e-6;
+  const double ps = 112.0 + 31.0 * std::min(std::max((mb - 64.0) / (127.0 - 64.0), 0.0), 1.0);
+  return 40e-6 + issued_flops / 820e12 < 18e-6 + (double)n_pairs * ps * 1e-12;
+}
 
 void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a, const double* b, double* c,
                     int parts) {
   MixedPlan& MP = get_mixed_plan(S, mult_type, ra, rb, rc);
   int k = S.mixed_kernel;
   if (parts == 3) k = 1;
-  if (k == 0 && !umma_usable(S, mult_type, ra, rb, rc)) k = 1;
+  if (k == 0 && !umma_usable(S)) k = 1;
   if (k < 0) {
     if (MP.kernel < 0) {
       MP.kernel = 1;
-      if (S.ranges[MP.out_range]->nnz >= kTileMinBlocks && umma_usable(S, mult_type, ra, rb, rc)) {
-        const UmmaPlan& U = get_umma_plan(S, mult_type, ra, rb, rc);
-        if (U.issued_flops > 0 && 3.0 * (double)U.flops / (double)U.issued_flops >= kTileMinFill) MP.kernel = 0;
-      }
+      if (MP.n_pairs >= kTileMinPairs && umma_usable(S) &&
+          split_tiles_pay(MP.n_pairs, MP.flops, umma_issued_estimate(S, mult_type, ra, rb, rc), S.ranges[rb]->nnz))
+        MP.kernel = 0;
     }
     k = MP.kernel;
   }

@@ -539,6 +539,109 @@ __global__ void k_umma_btab(int n_out, PlanDev D, const unsigned int* __restrict
 
 }  // namespace
 
+// The partition behind every tile plan of a system: contraction units and column chunks over the cover atoms (cover
+// order, the same for every row group) and row groups of consecutive primary atoms.
+namespace {
+struct CoverTiling {
+  std::vector<int> nd_prim;                         // block size of each primary atom
+  std::vector<int> unit_of, unit_pos;               // cover atom -> unit, position in it
+  std::vector<int> chunk_of, chunk_pos, chunk_first;
+  std::vector<unsigned int> ktab;                   // [unit][16]
+  std::vector<int> grp_first;                       // at most kM rows and kMaxAtoms atoms each
+  int n_units() const { return (int)(ktab.size() / kUK); }
+  int n_chunks() const { return (int)chunk_first.size() - 1; }
+  int n_groups() const { return (int)grp_first.size() - 1; }
+};
+
+CoverTiling cover_tiling(const Geometry& g) {
+  CoverTiling t;
+  const int np = g.n_prim, ncov = g.n_cover_atoms;
+  t.nd_prim.resize(np);
+  for (int p = 0; p < np; ++p) t.nd_prim[p] = g.nsf[g.prim_global[p]];
+  t.unit_of.resize(ncov); t.unit_pos.resize(ncov); t.chunk_of.resize(ncov); t.chunk_pos.resize(ncov);
+  int u = -1, uw = kUK + 1, ua = kMaxUnitAtoms;
+  for (int c = 0; c < ncov; ++c) {
+    const int nd = g.cover_nsf[c];
+    if (uw + nd > kUK || ua == kMaxUnitAtoms) { ++u; uw = 0; ua = 0; t.ktab.resize((size_t)(u + 1) * kUK, 0xffffffffu); }
+    for (int o = 0; o < nd; ++o) t.ktab[(size_t)u * kUK + uw + o] = (unsigned)ua | ((unsigned)o << 8) | ((unsigned)nd << 16);
+    t.unit_of[c] = u; t.unit_pos[c] = ua;
+    uw += nd; ++ua;
+  }
+  for (int c = 0, w = kNT + 1, cnt = kMaxAtoms; c < ncov; ++c) {
+    const int nd = g.cover_nsf[c];
+    if (w + nd > kNT || cnt == kMaxAtoms) { t.chunk_first.push_back(c); w = 0; cnt = 0; }
+    t.chunk_of[c] = (int)t.chunk_first.size() - 1;
+    t.chunk_pos[c] = cnt;
+    w += nd; ++cnt;
+  }
+  t.chunk_first.push_back(ncov);
+  for (int p = 0, rows = kM + 1, cnt = 0; p < np; ++p) {
+    if (rows + t.nd_prim[p] > kM || cnt == kMaxAtoms) { t.grp_first.push_back(p); rows = 0; cnt = 0; }
+    rows += t.nd_prim[p]; ++cnt;
+  }
+  t.grp_first.push_back(np);
+  return t;
+}
+
+// one warp per output block in [q0, q1): new (column chunk, unit) bits of its pairs are counted, and its pairs
+__global__ void k_umma_sample(int q0, int q1, const int64_t* __restrict__ ptr, const int2* __restrict__ pairs,
+                              const int* __restrict__ xcov, const int* __restrict__ ocov, const int* __restrict__ unit_of,
+                              const int* __restrict__ chunk_of, int n_units, unsigned int* __restrict__ bits,
+                              unsigned long long* __restrict__ counts) {
+  const int q = q0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (q >= q1) return;
+  const int64_t base = (int64_t)chunk_of[ocov[q]] * n_units;
+  unsigned n = 0;
+  for (int64_t p = ptr[q] + lane; p < ptr[q + 1]; p += 32) {
+    const int64_t bit = base + unit_of[xcov[pairs[p].x]];
+    const unsigned m = 1u << (bit & 31);
+    if (!(atomicOr(bits + (bit >> 5), m) & m)) ++n;
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) {
+    if (n) atomicAdd(counts, (unsigned long long)n);
+    atomicAdd(counts + 1, (unsigned long long)(ptr[q + 1] - ptr[q]));
+  }
+}
+}  // namespace
+
+// Tensor work that the tile plan of a product would issue, from up to twelve of its row groups (0: not known).  The plan
+// itself takes the host loops over every output block and tens of milliseconds on large products; this takes one pass over
+// the pairs of the sampled rows.
+double umma_issued_estimate(System& S, int mult_type, int ra, int rb, int rc) {
+  ProductPlan& P = get_plan(S, mult_type, ra, rb, rc);
+  RangeIndex& O = mult_type == 1 ? *S.ranges[rc] : *S.ranges[ra];
+  RangeIndex& X = mult_type == 1 ? *S.ranges[ra] : *S.ranges[rc];
+  if (O.nnz == 0 || !umma_usable(S)) return 0.0;
+  const CoverTiling ct = cover_tiling(S.geo);
+  const int ng = ct.n_groups(), ns = std::min(ng, 12);
+  const int64_t words = ((int64_t)ct.n_units() * ct.n_chunks() + 31) / 32;
+  if (words > (int64_t)1 << 28) return 0.0;         // 1 GiB of marks
+  cudaStream_t st = S.stream;
+  DevBuf<int> unit_of, chunk_of;
+  unit_of.upload(ct.unit_of, st);
+  chunk_of.upload(ct.chunk_of, st);
+  DevBuf<unsigned int> bits;
+  bits.alloc(words, st);
+  DevBuf<unsigned long long> counts;
+  counts.alloc(2, st);
+  CQ_CUDA(cudaMemsetAsync(counts.p, 0, 2 * sizeof(unsigned long long), st));
+  for (int k = 0; k < ns; ++k) {
+    const int gi = (int)((2 * (int64_t)k + 1) * ng / (2 * ns));
+    const int q0 = O.h_row_ptr[ct.grp_first[gi]], q1 = O.h_row_ptr[ct.grp_first[gi + 1]];
+    if (q0 == q1) continue;
+    CQ_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned int) * words, st));
+    k_umma_sample<<<(int)(((int64_t)(q1 - q0) * 32 + 255) / 256), 256, 0, st>>>(
+        q0, q1, P.ptr.p, P.pairs.p, X.nb_cover.p, O.nb_cover.p, unit_of.p, chunk_of.p, ct.n_units(), bits.p, counts.p);
+    CQ_CUDA(cudaGetLastError());
+    S.launches++;
+  }
+  unsigned long long c[2] = {0, 0};
+  CQ_CUDA(cudaMemcpyAsync(c, counts.p, sizeof(c), cudaMemcpyDeviceToHost, st));
+  CQ_CUDA(cudaStreamSynchronize(st));
+  return c[1] ? 3.0 * 2 * kM * kNT * kUK * (double)c[0] * (double)P.n_pairs / (double)c[1] : 0.0;
+}
+
 UmmaPlan& get_umma_plan(System& S, int mult_type, int ra, int rb, int rc) {
   auto key = std::make_tuple(mult_type, ra, rb, rc);
   auto it = S.uplans.find(key);
@@ -552,52 +655,21 @@ UmmaPlan& get_umma_plan(System& S, int mult_type, int ra, int rb, int rc) {
   RangeIndex& O = mult_type == 1 ? *S.ranges[rc] : *S.ranges[ra];
   RangeIndex& X = mult_type == 1 ? *S.ranges[ra] : *S.ranges[rc];
   const Geometry& g = S.geo;
-  const int np = g.n_prim, ncov = g.n_cover_atoms;
-  std::vector<int> nd_prim(np);
-  for (int p = 0; p < np; ++p) nd_prim[p] = g.nsf[g.prim_global[p]];
-  U.usable = true;
-  for (int p = 0; p < np; ++p) U.usable = U.usable && nd_prim[p] >= kMinNd && nd_prim[p] <= kUK;
-  for (int c = 0; c < ncov; ++c) U.usable = U.usable && g.cover_nsf[c] >= kMinNd && g.cover_nsf[c] <= kUK;
+  U.usable = umma_usable(S);
   if (!U.usable || O.nnz == 0) {
     auto res = S.uplans.emplace(key, std::move(up));
     return *res.first->second;
   }
-  // contraction units and column chunks over the cover atoms (cover order, the same for every row group)
-  std::vector<int> unit_of(ncov), unit_pos(ncov), chunk_of(ncov), chunk_pos(ncov), chunk_first;
-  std::vector<unsigned int> ktab;                   // [unit][16]
-  {
-    int u = -1, uw = kUK + 1, ua = kMaxUnitAtoms;
-    for (int c = 0; c < ncov; ++c) {
-      const int nd = g.cover_nsf[c];
-      if (uw + nd > kUK || ua == kMaxUnitAtoms) { ++u; uw = 0; ua = 0; ktab.resize((size_t)(u + 1) * kUK, 0xffffffffu); }
-      for (int o = 0; o < nd; ++o) ktab[(size_t)u * kUK + uw + o] = (unsigned)ua | ((unsigned)o << 8) | ((unsigned)nd << 16);
-      unit_of[c] = u; unit_pos[c] = ua;
-      uw += nd; ++ua;
-    }
-    int w = kNT + 1, cnt = kMaxAtoms;
-    for (int c = 0; c < ncov; ++c) {
-      const int nd = g.cover_nsf[c];
-      if (w + nd > kNT || cnt == kMaxAtoms) { chunk_first.push_back(c); w = 0; cnt = 0; }
-      chunk_of[c] = (int)chunk_first.size() - 1;
-      chunk_pos[c] = cnt;
-      w += nd; ++cnt;
-    }
-    chunk_first.push_back(ncov);
-  }
-  const int n_units = (int)(ktab.size() / kUK), n_chunks = (int)chunk_first.size() - 1;
+  CoverTiling ct = cover_tiling(g);
+  const std::vector<int>&nd_prim = ct.nd_prim, &chunk_first = ct.chunk_first, &grp_first = ct.grp_first;
+  std::vector<int>&unit_of = ct.unit_of, &unit_pos = ct.unit_pos, &chunk_of = ct.chunk_of, &chunk_pos = ct.chunk_pos;
+  std::vector<unsigned int>& ktab = ct.ktab;
+  const int n_units = ct.n_units(), n_chunks = ct.n_chunks(), ng = ct.n_groups();
   // host copies of the output and first-operand neighbour lists
   std::vector<int> ocov(O.nnz), xcov(std::max(X.nnz, 1));
   CQ_CUDA(cudaMemcpyAsync(ocov.data(), O.nb_cover.p, sizeof(int) * O.nnz, cudaMemcpyDeviceToHost, st));
   if (X.nnz) CQ_CUDA(cudaMemcpyAsync(xcov.data(), X.nb_cover.p, sizeof(int) * X.nnz, cudaMemcpyDeviceToHost, st));
   CQ_CUDA(cudaStreamSynchronize(st));
-  // row groups: consecutive primary atoms, at most kM rows and kMaxAtoms atoms
-  std::vector<int> grp_first;
-  for (int p = 0, rows = kM + 1, cnt = 0; p < np; ++p) {
-    if (rows + nd_prim[p] > kM || cnt == kMaxAtoms) { grp_first.push_back(p); rows = 0; cnt = 0; }
-    rows += nd_prim[p]; ++cnt;
-  }
-  grp_first.push_back(np);
-  const int ng = (int)grp_first.size() - 1;
   // row tables of the row groups (offset 128 g) and of the column chunks (offset 128 (ng + chunk))
   std::vector<unsigned int> rtabs((size_t)(ng + n_chunks) * kM, 0xffffffffu);
   for (int gi = 0; gi < ng; ++gi)
@@ -801,8 +873,10 @@ int* device_timeout_word(System& S) {
   return S.umma_err_dev;
 }
 
-bool umma_usable(System& S, int mult_type, int ra, int rb, int rc) {
-  return get_umma_plan(S, mult_type, ra, rb, rc).usable;
+bool umma_usable(const System& S) {
+  bool ok = true;
+  for (int v : S.geo.nsf) ok = ok && v >= kMinNd && v <= kUK;
+  return ok;
 }
 
 void mat_mult_umma(System& S, int mult_type, int ra, int rb, int rc, double* a, const double* b, double* c) {

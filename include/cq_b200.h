@@ -197,6 +197,11 @@ int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int
 int cq_product_tensor_work(cq_system* sys, int mult_type, int ra, int rb, int rc, int64_t* tiles,
                            int64_t* issued_flops, int* usable);
 
+/* The fixed rule by which a CQ_PREC_BF16X3 product takes the tcgen05 tiles (*kernel = 0) or one block per
+ * mma.sync warp (*kernel = 1), from its pairs and flops (cq_product_work), the tensor flops its tiles issue
+ * (cq_product_tensor_work; the library samples them) and the blocks of range rb.  Host-only, needs no GPU. */
+int cq_split_kernel_rule(int64_t n_pairs, int64_t flops, double issued_flops, int64_t b_blocks, int* kernel);
+
 /*
  * Drop-in kernel pair (plugin surface of multiply_kernel_<MULT_KERN>.f90):
  * the argument lists of m_kern_max / m_kern_min
@@ -287,8 +292,7 @@ int cq_generate_SH(cq_system* sys, int r, int which, uint64_t seed, double* out)
 #define CQ_OPT_BLOCKING_SYNC 2
 /* CQ_OPT_MIXED_KERNEL: kernel of the CQ_PREC_BF16X3 products (CQ_PREC_BF16X6 products always run on
  * mma.sync: the tcgen05 tiles accumulate a whole contraction in FP32).  -1 (default) = chosen per product
- * by a fixed rule (the tiles where at least 11 % of their issued tensor work is useful, from 2.5 million
- * output blocks on), so a product always gives the same bits; 0 = dense 128 x 128 tiles on the tcgen05 tensor cores with TMEM
+ * by a fixed rule on its counts (cq_split_kernel_rule), so a product always gives the same bits; 0 = dense 128 x 128 tiles on the tcgen05 tensor cores with TMEM
  * accumulators, operands staged by bulk copies (every block size 4..16; other systems use 1);
  * 1 = one padded 16 x 16 block per warp-level mma.sync. */
 #define CQ_OPT_MIXED_KERNEL 3

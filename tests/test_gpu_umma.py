@@ -147,6 +147,42 @@ def test_bounded_wait_reports_timeout_and_context_survives(cfg1):
     _assert_bound(got, ref, bound)
 
 
+@pytest.mark.parametrize("shape,mult_type,tiles", [("dense_dzp", 1, True), ("dense_dzp", 2, True), ("dense_mix", 1, True),
+                                                   ("dense_sz", 2, True), ("cell_dzp", 1, False), ("cell_sz", 2, False),
+                                                   ("small_dzp", 1, False)])
+def test_automatic_kernel_of_the_two_part_split(shape, mult_type, tiles):
+    """The automatic choice runs the kernel that the rule names for the product's counts (here with the issued flops of the
+    whole tile plan, where the library samples them): tiles on dense clusters, blocks on cells and on small products.  Both
+    kernels are held to their bounds elsewhere; the bits say which one ran."""
+    import torch
+    import cq_b200
+    kind, blocks = shape.split("_")
+    if kind == "cell":
+        coords, cell = inputs.diamond_si(2, sigma=0.1, seed=2)
+    else:
+        coords, cell = inputs.si_cluster(40 if kind == "small" else 100, sigma=0.1, seed=2, vacuum=15.0)
+    nd = {"dzp": lambda k: 13, "sz": lambda k: 4, "mix": lambda k: 13 if k % 3 == 0 else 4}[blocks]
+    g = cq_b200.System(coords, cell, np.array([nd(k) for k in range(len(coords))], np.int32), [20.0, 20.0, 40.0])
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7)
+    ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for r in range(3)]
+    o = 2 if mult_type == 1 else 0
+    outs = {}
+    for k in (-1, 0, 1):
+        g.set_mixed_kernel(k)
+        ops[o].fill_(float("nan"))
+        torch.cuda.synchronize()
+        g.mat_mult(mult_type, 0, 1, 2, *ops, precision=cq_b200.PREC_BF16X3)
+        g.synchronize()
+        outs[k] = ops[o].clone()
+    assert not torch.isnan(outs[-1]).any()
+    assert not torch.equal(outs[0], outs[1])
+    pairs, flops = g.product_work(mult_type, 0, 1, 2)
+    issued = g.product_tensor_work(mult_type, 0, 1, 2)[1]
+    assert cq_b200.split_kernel_rule(pairs, flops, issued, g.n_blocks(1)) == (0 if tiles else 1)
+    assert torch.equal(outs[-1], outs[0 if tiles else 1])
+
+
 # Three-part split (BF16x6): v = hi + mid + lo, six products per block pair, each pair's 16 x 16 x 16
 # product rounded to FP32 once and the pairs summed in FP64.  The omitted products and split
 # remainders are below 2^-23 |a||b| per element product and the FP32 rounding of a pair's product
