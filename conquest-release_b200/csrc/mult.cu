@@ -57,54 +57,73 @@ struct MultArgs {
 // Output block at a slot of the launch: the plan's order where it has been built, else the stored order.
 __device__ __forceinline__ int ordered(const int* __restrict__ order, int slot) { return order ? order[slot] : slot; }
 
-// Generic block sizes (nd <= 16): one warp per output block, up to 8 elements per lane.
-template <int TYPE, bool EXACT>
-__global__ void __launch_bounds__(256) k_mult_generic(MultArgs M) {
-  int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// Any block sizes (nd <= 16): one warp per output block, R elements per lane (32 R >= the largest block), operands read
+// from global memory.  What bounds it: the chain of dependent loads of a pair (pair list, block offsets, inner dimension,
+// values), so the next pair's offsets are looked up while the current one's values are on their way, and the list is read
+// a pair further ahead.  It is the kernel of small blocks in products with few output blocks, where the group kernel
+// waits for its staging (see auto_variant).  u: the block size when the whole system has one, else 0.
+// Measured (6298 output blocks, type 2, 47 terms each; us): 5 x 5 blocks 50.3, without the look-ahead 99.5 and 113.2
+// for the group kernel; blocks of 1 and 4 rows 55.6, 76.0 and 86.2.
+template <int TYPE, bool EXACT, int R>
+__global__ void __launch_bounds__(256) k_mult_generic(MultArgs M, int u) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (q >= M.n_out) return;
-  const int ndi = M.prim_nsf[M.o_row[q]];
-  const int ndo = M.cover_nsf[M.o_cover[q]];    // type 1: nd_j ; type 2: nd_k
+  const int2* pairs = M.pairs + M.ptr[q];
+  const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
+  const int ndi = u ? u : M.prim_nsf[M.o_row[q]];
+  const int ndo = u ? u : M.cover_nsf[M.o_cover[q]];    // type 1: nd_j ; type 2: nd_k
   const int ne = ndi * ndo;
-  double acc[8];
+  double acc[R];
+  int n1[R], n2[R];                             // row and column of the lane's elements
 #pragma unroll
-  for (int r = 0; r < 8; ++r) acc[r] = 0.0;
-  const int64_t p0 = M.ptr[q], p1 = M.ptr[q + 1];
-  for (int64_t t = p0; t < p1; ++t) {
-    int2 pr = __ldcs(M.pairs + t);
-    const double* X = M.x + M.x_elem[pr.x];
-    const double* B = M.b + M.b_elem[pr.y];
-    if (TYPE == 1) {
-      const int ndk = M.cover_nsf[M.x_cover[pr.x]];
+  for (int r = 0; r < R; ++r) {
+    const int e = min(lane + 32 * r, ne - 1);   // clamped: in-bounds reads
+    n2[r] = e / ndi;
+    n1[r] = e - ndi * n2[r];
+    acc[r] = 0.0;
+  }
+  struct Term { const double *x, *b; int nk; };
+  auto look_up = [&](int2 pr) {
+    Term v;
+    v.x = M.x + (u ? (int64_t)pr.x * (u * u) : M.x_elem[pr.x]);
+    v.b = M.b + (u ? (int64_t)pr.y * (u * u) : M.b_elem[pr.y]);
+    v.nk = u ? u : TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]];
+    return v;
+  };
+  Term next = {nullptr, nullptr, 0};
+  int2 pn = make_int2(0, 0);
+  if (nt > 0) next = look_up(__ldcs(pairs));
+  if (nt > 1) pn = __ldcs(pairs + 1);
+  for (int t = 0; t < nt; ++t) {
+    const Term cur = next;
+    if (t + 1 < nt) next = look_up(pn);
+    if (t + 2 < nt) pn = __ldcs(pairs + t + 2);
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        int e = lane + 32 * r;
-        if (e < ne) {
-          int n1 = e % ndi, n2 = e / ndi;
-          double a = acc[r];
-          for (int n3 = 0; n3 < ndk; ++n3) a = madd<EXACT>(a, X[n1 + ndi * n3], B[n3 + ndk * n2]);
-          acc[r] = a;
-        }
+    for (int r = 0; r < R; ++r) {
+      if (R > 1 && 32 * r >= ne) break;
+      // type 1: a(n1, n) b(n, n2); type 2: c(n1, n) b(n2, n)
+      const double *x = cur.x + n1[r], *b = cur.b + (TYPE == 1 ? cur.nk * n2[r] : n2[r]);
+      double a = acc[r];
+      if constexpr (R <= 2) {                   // blocks of at most K rows and columns: one batch of loads
+        constexpr int K = R == 1 ? 5 : 8;
+        double xv[K], bv[K];
+#pragma unroll
+        for (int n = 0; n < K; ++n)
+          if (n < cur.nk) { xv[n] = __ldg(x + ndi * n); bv[n] = __ldg(b + (TYPE == 1 ? n : ndo * n)); }
+#pragma unroll
+        for (int n = 0; n < K; ++n)
+          if (n < cur.nk) a = madd<EXACT>(a, xv[n], bv[n]);
+      } else {
+#pragma unroll 4
+        for (int n = 0; n < cur.nk; ++n) a = madd<EXACT>(a, __ldg(x + ndi * n), __ldg(b + (TYPE == 1 ? n : ndo * n)));
       }
-    } else {
-      const int ndj = M.cover_nsf[M.b_cover[pr.y]];
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        int e = lane + 32 * r;
-        if (e < ne) {
-          int n1 = e % ndi, n3 = e / ndi;
-          double a = acc[r];
-          for (int n2 = 0; n2 < ndj; ++n2) a = madd<EXACT>(a, X[n1 + ndi * n2], B[n3 + ndo * n2]);
-          acc[r] = a;
-        }
-      }
+      acc[r] = a;
     }
   }
   double* O = M.out + M.o_elem[q];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    int e = lane + 32 * r;
-    if (e < ne) O[e] = acc[r];
-  }
+  for (int r = 0; r < R; ++r)
+    if (lane + 32 * r < ne) O[lane + 32 * r] = acc[r];
 }
 
 // 4 x 4 blocks (SZ basis): 16 lanes per output block, one element per lane.  Each lane
@@ -1320,12 +1339,18 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) by_size(integral_constant<int, 2>{}, std::true_type{}); else by_size(integral_constant<int, 2>{}, std::false_type{});
     }
   } else {
-    int grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
-    if (P.mult_type == 1) {
-      if (exact) k_mult_generic<1, true><<<grid, T, 0, st>>>(M); else k_mult_generic<1, false><<<grid, T, 0, st>>>(M);
-    } else {
-      if (exact) k_mult_generic<2, true><<<grid, T, 0, st>>>(M); else k_mult_generic<2, false><<<grid, T, 0, st>>>(M);
-    }
+    const int grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
+    auto by_type = [&](auto r) {
+      constexpr int R = decltype(r)::value;
+      if (P.mult_type == 1) {
+        if (exact) k_mult_generic<1, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf); else k_mult_generic<1, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+      } else {
+        if (exact) k_mult_generic<2, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf); else k_mult_generic<2, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+      }
+    };
+    if (S.max_nsf <= 5) by_type(std::integral_constant<int, 1>{});
+    else if (S.max_nsf <= 8) by_type(std::integral_constant<int, 2>{});
+    else by_type(std::integral_constant<int, 8>{});
   }
   S.launches++;
   CQ_CUDA(cudaGetLastError());
@@ -1341,11 +1366,15 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
 //    248 / 316; 24,064: 472 / 378 / 322); above, the row kernel, whose steps are the rows of B: where the lists
 //    hold most of those rows, and from 40,000 blocks on (every SM full) also most lanes have a block (63,664 with
 //    97 % of the lanes: 605 / 823 / 570; 47,000 with 73 %: 520 / 625 / 611; lists of 88 %: 127 / 170 / 135).
-// Other block sizes and unaligned operands: the group kernel (the generic one is 3 to 5 times slower).
+// Other block sizes and unaligned operands: the group kernel (on 13 x 13 blocks the generic one is 2 to 3 times slower),
+// except for small blocks in few output blocks, whose time is the latency of a step and not its arithmetic (generic /
+// group, us): blocks of up to 5 rows below 17,000 output blocks (1600 of 1 and 4 rows 11.9 / 22.5; 6298 55.6 / 86.2; 15,342
+// equal; 71,030 67.3 / 60.9), of 6 to 8 below 2,000 (1862 of 8 x 8 43.6 / 60.2; 3016 86 / 100 in the group's favour).
 static int auto_variant(System& S, ProductPlan& P, int n_out, bool nd4) {
   if (!nd4) {
-    if (S.uniform_nsf != 4) P.tuned = 4;
-    return 4;
+    const int variant = n_out < (S.max_nsf <= 5 ? 17000 : S.max_nsf <= 8 ? 2000 : 0) ? 0 : 4;
+    if (S.uniform_nsf != 4) P.tuned = variant;
+    return variant;
   }
   if (P.tuned >= 0) return P.tuned;
   if (P.mult_type == 1) return P.tuned = n_out < 180000 ? 5 : 3;
