@@ -84,24 +84,39 @@ __global__ void __launch_bounds__(kT) k_masked_add_nd4(int nnz, const int* __res
     a[i] = x;
   }
 }
-// AT(dest) = A(e)^T: a warp per block, through shared memory so that both the read and the write run along memory
+// AT(dest) = A(e)^T: a warp per block.  STAGED: through shared memory, so that both the read and the write run along
+// memory; else each lane writes its elements where they belong, one round trip less (see dev_transpose).
+template <bool STAGED>
 __global__ void __launch_bounds__(kT) k_transpose(int nnz, const int* __restrict__ dest, const int64_t* __restrict__ elem,
                                                   const int* __restrict__ row, const int* __restrict__ cover,
                                                   const int* __restrict__ prim_nsf, const int* __restrict__ cover_nsf,
                                                   const double* __restrict__ a, double* __restrict__ at) {
-  __shared__ double tile[kT / 32][256];
   int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e >= nnz) return;
-  int ndi = prim_nsf[row[e]], ndj = cover_nsf[cover[e]];
+  const int ndi = prim_nsf[row[e]], ndj = cover_nsf[cover[e]], ne = ndi * ndj;
   const double* A = a + elem[e];
   double* T = at + elem[dest[e]];
-  double* W = tile[threadIdx.x >> 5];
-  const int ne = ndi * ndj, magic = 65536 / ndj + 1;      // t / ndj = t * magic >> 16 for t < 256, ndj <= 16
-  for (int t = lane; t < ne; t += 32) W[t] = A[t];
-  __syncwarp();
-  for (int t = lane; t < ne; t += 32) {                   // element (n2, n1) of the transpose
-    const int n1 = (t * magic) >> 16, n2 = t - n1 * ndj;
-    T[t] = W[n1 + ndi * n2];
+  if constexpr (STAGED) {
+    __shared__ double tile[kT / 32][16 * 17];
+    double* W = tile[threadIdx.x >> 5];
+    const int pad = ~ndi & 1, ld = ndi + pad;              // odd column distance: the reads along a row hit different banks
+    const int by_j = 65536 / ndj + 1;                      // t / ndj = t * by_j >> 16 for t < 256, ndj <= 16
+    if (pad) {
+      const int by_i = 65536 / ndi + 1;
+      for (int t = lane; t < ne; t += 32) W[t + ((t * by_i) >> 16)] = A[t];
+    } else {
+      for (int t = lane; t < ne; t += 32) W[t] = A[t];
+    }
+    __syncwarp();
+    for (int t = lane; t < ne; t += 32) {                  // element (n2, n1) of the transpose
+      const int n1 = (t * by_j) >> 16, n2 = t - n1 * ndj;
+      T[t] = W[n1 + ld * n2];
+    }
+  } else {
+    for (int t = lane; t < ne; t += 32) {
+      const int n1 = t % ndi, n2 = t / ndi;
+      T[n2 + ndj * n1] = A[t];
+    }
   }
 }
 // the same for uniform 4 x 4 blocks with 16-byte aligned arrays: eight lanes per block; lane (n1 pair, n2) reads two
@@ -371,9 +386,14 @@ void dev_transpose(System& S, int r, const double* a, double* at) {
   if (S.uniform_nsf == 4 && ((uintptr_t)a | (uintptr_t)at) % 16 == 0)
     k_transpose_nd4<<<grid_for((int64_t)R.nnz * 8), kT, 0, S.stream>>>(
         R.nnz, R.trans_dest.p, reinterpret_cast<const double2*>(a), reinterpret_cast<double2*>(at));
-  else
-    k_transpose<<<(int)(((int64_t)R.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
+  else {
+    // staged from a mean of 110 elements per block on (512 atoms, 16-bohr range, staged / direct, us): 13 x 13 36.4 / 45.0,
+    // 16 x 16 44.6 / 74.7 (79.0 before its columns were padded in shared memory), 11 x 11 34.7 / 35.6, 10 x 10 31.3 / 24.9,
+    // 4 and 13 rows 14.7 / 12.5, 1 and 4 rows 12.1 / 8.9
+    auto* kern = R.length >= (int64_t)110 * R.nnz ? k_transpose<true> : k_transpose<false>;
+    kern<<<(int)(((int64_t)R.nnz * 32 + kT - 1) / kT), kT, 0, S.stream>>>(
         R.nnz, R.trans_dest.p, R.nb_elem.p, R.nb_row.p, R.nb_cover.p, S.dg.prim_nsf.p, S.dg.cover_nsf.p, a, at);
+  }
   S.launches++;
   CQ_CUDA(cudaGetLastError());
 }
