@@ -333,7 +333,7 @@ void pinned_put(uint64_t* p);
 
 // index.cu
 void upload_geometry(System& S);
-int64_t dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st);   // out[0..n], returns the total
+void dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st);   // out[0..n], enqueued
 void build_range_index(System& S, RangeIndex& R);
 ProductPlan& get_plan(System& S, int mult_type, int ra, int rb, int rc);
 AddMap& get_addmap(System& S, int ra, int rb);

@@ -384,9 +384,9 @@ __global__ void k_scan_add(int64_t* __restrict__ out, int64_t n, const int64_t* 
   if (i < n) out[i] += s[blockIdx.x];
 }
 
-// exclusive scan of n values into out[0..n]; out[n] = total.  Returns the total (synchronises).
+// exclusive scan of n values into out[0..n]; out[n] = total
 template <class Tin>
-int64_t exclusive_scan(const Tin* in, int64_t n, int64_t* out, cudaStream_t st) {
+void enqueue_scan(const Tin* in, int64_t n, int64_t* out, cudaStream_t st) {
   int nb = (int)std::max<int64_t>(1, (n + 255) / 256);
   DevBuf<int64_t> sums;
   sums.alloc(nb + 1, st);
@@ -395,6 +395,11 @@ int64_t exclusive_scan(const Tin* in, int64_t n, int64_t* out, cudaStream_t st) 
   k_scan_sums<<<1, 1024, 0, st>>>(sums.p, n > 0 ? nb : 0, out + n);
   if (n > 0) k_scan_add<<<nb, 256, 0, st>>>(out, n, sums.p);
   CQ_CUDA(cudaGetLastError());
+}
+// the same; returns the total (synchronises)
+template <class Tin>
+int64_t exclusive_scan(const Tin* in, int64_t n, int64_t* out, cudaStream_t st) {
+  enqueue_scan(in, n, out, st);
   int64_t total = 0;
   CQ_CUDA(cudaMemcpyAsync(&total, out + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CQ_CUDA(cudaStreamSynchronize(st));
@@ -423,7 +428,7 @@ int read_flag(int* d, cudaStream_t st) {
 
 }  // namespace
 
-int64_t dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st) { return exclusive_scan(in, n, out, st); }
+void dev_exclusive_scan(const int* in, int64_t n, int64_t* out, cudaStream_t st) { enqueue_scan(in, n, out, st); }
 
 void upload_geometry(System& S) {
   Geometry& g = S.geo;

@@ -1030,6 +1030,77 @@ __global__ void __launch_bounds__(64) k_mult_dmma(MultArgs M, const int* __restr
   for (int e = lane; e < ndi * ndo; e += 32) __stcs(D + e, O[e]);
 }
 
+// The same MMAs for short lists: one warp per output block in the stored order, one pair at a time, the operands read
+// straight from the block storage into fragments (the next pair's while the current one's MMAs run), no shared memory.
+// What bounds it is that chain of loads; it is the faster one where a list is a round or two long (dmma_short).
+template <int TYPE>
+__device__ __forceinline__ void dmma_load_pair(const MultArgs& M, int2 pr, int ndi, int ndo, int g, int t,
+                                               double (&av)[4][2], double (&bv)[4][2], int& nks) {
+  const double* X = M.x + M.x_elem[pr.x];
+  const double* B = M.b + M.b_elem[pr.y];
+  const int nk = TYPE == 1 ? M.cover_nsf[M.x_cover[pr.x]] : M.cover_nsf[M.b_cover[pr.y]];
+  nks = (nk + 3) >> 2;
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) {
+    const int n = 4 * ks + t;
+    const bool in = n < nk;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = 8 * h + g;                     // row of the first operand's fragment, column of B's
+      av[ks][h] = in && e < ndi ? __ldg(X + e + ndi * n) : 0.0;
+      bv[ks][h] = in && e < ndo ? __ldg(TYPE == 1 ? B + n + nk * e : B + e + ndo * n) : 0.0;
+    }
+  }
+}
+
+template <int TYPE>
+__global__ void __launch_bounds__(128) k_mult_dmma_short(MultArgs M) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= M.n_out) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int2* pairs = M.pairs + M.ptr[q];
+  const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
+  const int ndi = M.prim_nsf[M.o_row[q]];
+  const int ndo = M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
+  const bool rt = ndi > 8, ct = ndo > 8;         // a second row / column tile
+  double acc[2][2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  double av[4][2], bv[4][2];
+  int nks = 0;
+  if (nt > 0) dmma_load_pair<TYPE>(M, __ldcs(pairs), ndi, ndo, g, t, av, bv, nks);
+  for (int p = 0; p < nt; ++p) {
+    double nav[4][2], nbv[4][2];
+    int nnks = 0;
+    if (p + 1 < nt) dmma_load_pair<TYPE>(M, __ldcs(pairs + p + 1), ndi, ndo, g, t, nav, nbv, nnks);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      if (ks < nks) {
+        dmma_8x8x4(acc[0][0], av[ks][0], bv[ks][0]);
+        if (ct) dmma_8x8x4(acc[0][1], av[ks][0], bv[ks][1]);
+        if (rt) dmma_8x8x4(acc[1][0], av[ks][1], bv[ks][0]);
+        if (rt && ct) dmma_8x8x4(acc[1][1], av[ks][1], bv[ks][1]);
+      }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) { av[ks][h] = nav[ks][h]; bv[ks][h] = nbv[ks][h]; }
+    nks = nnks;
+  }
+  double* O = M.out + M.o_elem[q];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = 8 * i + g, c = 8 * j + 2 * t + e;
+        if (r < ndi && c < ndo) O[r + ndi * c] = acc[i][j][e];
+      }
+}
+
 // Many independent products in one persistent launch (the concatenation of their output-block
 // lists): every warp takes work units u = warp id, warp id + warps in the grid, ...; a unit is 32
 // output slots of a uniform 4 x 4 product (the warp-staged kernel) or two output blocks of any other
@@ -1187,7 +1258,7 @@ static bool capturing(const System& S) {
   return status != cudaStreamCaptureStatusNone;
 }
 
-// The plan's output order, built on its first use, which allocates and waits for the stream: a launch that is being
+// The plan's output order, built on its first use, which allocates: a launch that is being
 // captured into a graph before then runs in the stored order instead (null: the same results).
 static const int* output_order(System& S, ProductPlan& P) {
   const RangeIndex& O = *S.ranges[P.out_range];
@@ -1207,7 +1278,7 @@ static const int* output_order(System& S, ProductPlan& P) {
   first.alloc((size_t)bins * tiles + 1, S.stream);
   k_order_count<<<tiles, 256, bins * sizeof(int), S.stream>>>(key, O.nnz, bins, hist.p);
   CQ_CUDA(cudaGetLastError());
-  dev_exclusive_scan(hist.p, (int64_t)bins * tiles, first.p, S.stream);
+  dev_exclusive_scan(hist.p, (int64_t)bins * tiles, first.p, S.stream);   // nothing here waits for the device
   P.order.alloc(O.nnz, S.stream);
   k_order_fill<<<tiles, 256, bins * sizeof(int), S.stream>>>(key, O.nnz, bins, first.p, P.order.p);
   S.launches += 2;
@@ -1389,6 +1460,16 @@ static int auto_variant(System& S, ProductPlan& P, int n_out, bool nd4) {
   return P.tuned = n_out < 40000 ? (lists >= 0.75 ? 4 : 3) : (lists >= 0.9 && lanes >= 0.8 ? 4 : 3);
 }
 
+// FP64 tensor-core products whose time is latency: the short-list kernel, without an output order.  Not for one block size
+// of 13 (compiled in) or sizes up to 8 (one MMA tile per block), where the staged kernel is the faster one at every size.
+// Measured (staged / short, us): 4 and 13 rows, 3008 output blocks of 0.5 terms 6.0 / 5.5, 1600 of 12 19.1 / 16.0, 8070 of
+// 3.8 14.8 / 19.2, 2078 of 28 24.7 / 27.1; 5 and 13 rows, 2078 of 0.7 6.3 / 4.7, 4530 of 4.0 15.1 / 14.2, 10,100 of 3.1
+// 18.1 / 23.6; 16 x 16 blocks, 1600 of 12 37.5 / 23.8, 6288 of 9.3 51.5 / 47.5, 12,900 of 8.1 77.8 / 76.7, 3406 of 31 67.2 / 77.9.
+static bool dmma_short(const System& S, const ProductPlan& P, int n_out) {
+  if (S.uniform_nsf == 13 || S.max_nsf <= 8) return false;
+  return S.max_nsf <= 13 ? n_out < 5000 && P.n_pairs < 50000 : P.n_pairs < 100000;
+}
+
 // kernel arguments of one product (roles of mat_mult: type 1 writes c from a, b; type 2 writes a from c, b);
 // nd4: uniform 4 x 4 blocks with 16-byte aligned operands (the 4 x 4 kernels read 16-byte vectors)
 static MultArgs product_args(System& S, ProductPlan& P, double* a, const double* b, double* c, bool* nd4) {
@@ -1426,16 +1507,23 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   // those of the CUDA-core kernels (checked on B200), about three times faster on 13 x 13 blocks
   // (unless a CUDA-core variant is forced with CQ_OPT_MULT_VARIANT)
   if (exact == kPrecFp64Tensor || (exact == 0 && S.max_nsf > 8 && S.mult_variant == kVariantAuto)) {
-    const int* order = output_order(S, P);
-    const int grid = (M.n_out + 1) / 2;
-    if (P.mult_type == 1) {
-      if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, order);
-      else if (S.max_nsf <= 13) k_mult_dmma<1, 0, 13><<<grid, 64, 0, st>>>(M, order);
-      else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, order);
+    if (dmma_short(S, P, M.n_out)) {
+      const int grid = (M.n_out + 3) / 4;
+      if (P.mult_type == 1) k_mult_dmma_short<1><<<grid, 128, 0, st>>>(M);
+      else k_mult_dmma_short<2><<<grid, 128, 0, st>>>(M);
     } else {
-      if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, order);
-      else if (S.max_nsf <= 13) k_mult_dmma<2, 0, 13><<<grid, 64, 0, st>>>(M, order);
-      else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, order);
+      // below 1,200 output blocks every SM holds its share at once: the order would cost a first call more than it gives
+      const int* order = M.n_out < 1200 ? nullptr : output_order(S, P);
+      const int grid = (M.n_out + 1) / 2;
+      if (P.mult_type == 1) {
+        if (S.uniform_nsf == 13) k_mult_dmma<1, 13, 13><<<grid, 64, 0, st>>>(M, order);
+        else if (S.max_nsf <= 13) k_mult_dmma<1, 0, 13><<<grid, 64, 0, st>>>(M, order);
+        else k_mult_dmma<1, 0, 16><<<grid, 64, 0, st>>>(M, order);
+      } else {
+        if (S.uniform_nsf == 13) k_mult_dmma<2, 13, 13><<<grid, 64, 0, st>>>(M, order);
+        else if (S.max_nsf <= 13) k_mult_dmma<2, 0, 13><<<grid, 64, 0, st>>>(M, order);
+        else k_mult_dmma<2, 0, 16><<<grid, 64, 0, st>>>(M, order);
+      }
     }
     S.launches++;
     CQ_CUDA(cudaGetLastError());
