@@ -1304,7 +1304,8 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   RangeIndex& X = P.mult_type == 1 ? *S.ranges[P.ra] : *S.ranges[P.rc];
   // the row kernel's tiles are uploaded on its first use: a launch captured before then takes the warp-staged kernel
   if (nd4 && variant == 4 && P.mult_type == 2 && P.n_row_tiles < 0 && capturing(S)) variant = 3;
-  const int* order = nd4 && variant >= 3 ? output_order(S, P) : nullptr;
+  const bool row_kernel = nd4 && variant == 4 && P.mult_type == 2;        // the row kernel has an order of its own
+  const int* order = nd4 && variant >= 3 && !row_kernel ? output_order(S, P) : nullptr;
   if (nd4 && variant == 6) {
     const int grid = (M.n_out + 127) / 128;
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
@@ -1327,7 +1328,7 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) k_mult_nd4_quad<2, true, 4><<<grid, 128, 0, st>>>(M, order);
       else k_mult_nd4_quad<2, false, 4><<<grid, 128, 0, st>>>(M, order);
     }
-  } else if (nd4 && variant == 4 && P.mult_type == 2) {
+  } else if (row_kernel) {
     if (P.n_row_tiles < 0) {
       // up to 32 output blocks whose column atoms are images of one atom, with that atom's row of B
       RangeIndex& B = *S.ranges[P.rb];

@@ -185,3 +185,19 @@ def test_transposes_of_every_block_size(sizes):
         g.synchronize()
         assert np.array_equal(at.cpu().numpy(), bm.kat_transpose(bl, v))
         assert torch.equal(back, a)
+
+
+def test_row_kernel_builds_no_output_order():
+    """The type-2 4 x 4 row kernel walks rows of B, not the output order: its first call launches one kernel."""
+    import torch
+    import cq_b200
+    coords, cell = inputs.si_cluster(33, sigma=0.1, seed=95)
+    g = cq_b200.System(coords, cell, np.full(len(coords), 4, np.int32), [10.0, 8.0, 18.0])
+    ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda") for r in range(3)]
+    torch.cuda.synchronize()
+    g.product_work(2, 0, 1, 2)
+    g.set_mult_variant(4)
+    before = g.launch_count()
+    g.mat_mult(2, 0, 1, 2, *ops)
+    g.synchronize()
+    assert g.launch_count() - before == 1
