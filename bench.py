@@ -906,14 +906,17 @@ def mult_main(args):
                 ms.append(e0.elapsed_time(e1))
             m = float(np.median(ms))
             nbytes = 8.0 * (g.length(ra) + g.length(rb) + g.length(rc))
-            tv, tms = g.product_tuning(t, ra, rb, rc, mixed=(args.precision in ("bf16x3", "bf16x6")))
+            split = args.precision in ("bf16x3", "bf16x6")
+            tv, _ = g.product_tuning(t, ra, rb, rc, mixed=split)
             tensor = None
-            if args.precision == "bf16x3" and args.mixed_kernel != 1:
+            if split and tv == 0:          # the tcgen05 tiles ran
                 nt, issued, usable = g.product_tensor_work(t, ra, rb, rc)
                 tensor = {"tiles": nt, "issued_tflop": issued / 1e12, "useful_fraction": 3.0 * flops / max(issued, 1),
                           "issued_tflops": issued / (m / 1e3) / 1e12}
-            out.append({"product": name, "triples": triples, "flops": flops, "ms": m, "tuned_variant": tv,
-                        "tune_ms": tms, "tensor": tensor,
+            out.append({"product": name, "triples": triples, "flops": flops, "ms": m,
+                        "kernel": ("tcgen05 tiles" if tv == 0 else "mma.sync blocks") if split else
+                                  "variant %d" % tv if tv >= 0 else args.precision,
+                        "tensor": tensor,
                         "tflops": flops / (m / 1e3) / 1e12, "gbs_algorithmic": nbytes / (m / 1e3) / 1e9})
     tot_fl = sum(o["flops"] for o in out)
     tot_ms = sum(o["ms"] for o in out)

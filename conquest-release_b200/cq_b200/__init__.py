@@ -293,8 +293,8 @@ class System:
         return t.value, f.value
 
     def product_tuning(self, mult_type, ra, rb, rc, mixed=False):
-        """FP64: (variant chosen by the rule on sizes or -1, {variant: timed ms}); mixed=True: (output blocks per
-        warp of the split-precision kernel or -1 before its first call, {})."""
+        """FP64: (variant chosen by the rule on sizes or -1, {}); mixed=True: (output blocks per warp of the kernel that
+        the last split-precision call ran: 1 = mma.sync, 0 = the tcgen05 tiles, -1 before the first call, {})."""
         v, g = c_int(), c_int()
         ms, gms = (ctypes.c_float * 7)(), (ctypes.c_float * 4)()
         check(lib().cq_product_tuning(self._h, mult_type, ra, rb, rc, ctypes.byref(v), ms, ctypes.byref(g), gms))
@@ -349,7 +349,7 @@ class System:
     def set_mult_variant(self, v):
         """FP64 4x4 product kernel: -1 = chosen per product by size (default), 0 = one lane per output element,
         1 = one thread per output block, 2 = operand row staged in shared memory, 3 = warp-staged operand blocks,
-        5 = four lanes per output block, 6 = operand blocks staged by bulk copies."""
+        4 = for mult type 2, 3 with the shared row of B staged once, 5 = four lanes per output block, 6 = operand blocks staged by bulk copies."""
         check(lib().cq_system_set_option(self._h, 1, int(v)))
 
     def profile(self, on=True):

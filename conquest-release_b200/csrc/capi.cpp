@@ -321,9 +321,9 @@ int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int
     check_sys(sys); check_range(sys, ra); check_range(sys, rb); check_range(sys, rc);
     ProductPlan& P = get_plan(sys->S, mult_type, ra, rb, rc);
     if (variant) *variant = P.tuned;
-    if (ms) for (int v = 0; v < 7; ++v) ms[v] = P.tune_ms[v];
-    // one output block per warp in every split-precision product that has run
-    if (group) *group = sys->S.mplans.count(std::make_tuple(mult_type, ra, rb, rc)) ? 1 : -1;
+    if (ms) for (int v = 0; v < 7; ++v) ms[v] = 0.f;
+    const auto it = sys->S.mplans.find(std::make_tuple(mult_type, ra, rb, rc));
+    if (group) *group = it == sys->S.mplans.end() || it->second->last < 0 ? -1 : it->second->last;
     if (group_ms) for (int g = 0; g < 4; ++g) group_ms[g] = 0.f;
   });
 }

@@ -211,13 +211,13 @@ struct ProductPlan {
   DevBuf<int4> row_tiles;
   DevBuf<int> order;              // output blocks by descending pair count (staged kernels)
   int tuned = -1;                 // FP64 kernel variant chosen by auto_variant (-1: not chosen yet)
-  float tune_ms[7] = {0, 0, 0, 0, 0, 0, 0};
 };
 
 // Split-precision tensor-core product: pair lists sorted by the first operand block (one warp per output block).
 struct MixedPlan {
   int mult_type = 1, ra = -1, rb = -1, rc = -1, out_range = -1;
   int kernel = -1;                  // 0 = tcgen05 tiles, 1 = per-block mma.sync (-1: not chosen yet)
+  int last = -1;                    // kernel of the product's last call
   int64_t n_pairs = 0, flops = 0;
   DevBuf<int64_t> own_ptr;        // type 2 only (type 1 uses the FP64 plan's lists, already sorted)
   DevBuf<int2> own_pairs;

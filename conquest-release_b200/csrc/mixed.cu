@@ -355,6 +355,7 @@ void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a,
     }
     k = MP.kernel;
   }
+  MP.last = k;
   if (k == 0) mat_mult_umma(S, mult_type, ra, rb, rc, a, b, c);
   else mat_mult_mma_sync(S, MP, mult_type, ra, rb, rc, a, b, c, parts);
 }

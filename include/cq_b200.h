@@ -183,9 +183,9 @@ int cq_grab_matrix(cq_system* sys, int r, double* a_dev, const char* path, int64
 int cq_product_work(cq_system* sys, int mult_type, int ra, int rb, int rc, int64_t* triples, int64_t* flops);
 
 /* Kernel record of one product: the FP64 kernel variant chosen for it (-1 before the product's
- * first call with the automatic choice) and the timed milliseconds of each variant (ms[7], 0 = not
- * timed; the FP64 choice is a rule and times none); for its split-precision form the output blocks per
- * warp (1; -1 = has not run yet) and the timed milliseconds of four group sizes (group_ms[4], 0). */
+ * first call with the automatic choice); for its split-precision form the output blocks per warp of
+ * the kernel that its last call ran (1 = one per mma.sync warp, 0 = the tcgen05 tiles, -1 = has not run
+ * yet).  ms[7] and group_ms[4] are kept for existing callers and filled with zeros: nothing is timed. */
 int cq_product_tuning(cq_system* sys, int mult_type, int ra, int rb, int rc, int* variant, float* ms, int* group,
                       float* group_ms);
 

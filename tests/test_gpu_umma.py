@@ -168,6 +168,7 @@ def test_automatic_kernel_of_the_two_part_split(shape, mult_type, tiles):
     ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for r in range(3)]
     o = 2 if mult_type == 1 else 0
     outs = {}
+    assert g.product_tuning(mult_type, 0, 1, 2, mixed=True)[0] == -1
     for k in (-1, 0, 1):
         g.set_mixed_kernel(k)
         ops[o].fill_(float("nan"))
@@ -175,6 +176,10 @@ def test_automatic_kernel_of_the_two_part_split(shape, mult_type, tiles):
         g.mat_mult(mult_type, 0, 1, 2, *ops, precision=cq_b200.PREC_BF16X3)
         g.synchronize()
         outs[k] = ops[o].clone()
+        if k >= 0:
+            assert g.product_tuning(mult_type, 0, 1, 2, mixed=True)[0] == k          # the kernel of the last call
+        else:
+            assert g.product_tuning(mult_type, 0, 1, 2, mixed=True)[0] == (0 if tiles else 1)
     assert not torch.isnan(outs[-1]).any()
     assert not torch.equal(outs[0], outs[1])
     pairs, flops = g.product_work(mult_type, 0, 1, 2)
@@ -232,7 +237,8 @@ def test_three_part_split_mixed_sizes_within_bound():
 
 @pytest.mark.parametrize("precision_name", ["PREC_BF16X3", "PREC_BF16X6"])
 def test_split_group_sizes_give_the_same_bits(cfg1, precision_name):
-    """The mma.sync split kernels with 1, 2, 4 (and 8) output blocks per warp: the same bits."""
+    """CQ_OPT_SPLIT_GROUP is accepted for existing callers and changes no bit (it has no effect: the split kernels run one
+    output block per warp; they are held to their bounds on short lists and ragged sizes in test_gpu_edges.py)."""
     import cq_b200
     o, g, bls = cfg1
     prec = getattr(cq_b200, precision_name)
