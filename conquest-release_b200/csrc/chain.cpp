@@ -333,7 +333,7 @@ LNVSolver::~LNVSolver() {
 }
 
 // One LNV_matrix_multiply call.  With prm.graphs, the first call with a given set of operands runs
-// directly (it builds and tunes the products' plans and allocates their buffers), the second is
+// directly (it builds the products' plans and allocates their buffers), the second is
 // captured into a CUDA graph, and later ones replay that graph: one launch instead of ~60.
 void LNVSolver::lnv(bool doK, bool doM3, bool dophi, bool doE, DMat* M3, DMat* phim, double* electrons, double* energy) {
   ensure_workspace();

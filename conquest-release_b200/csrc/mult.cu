@@ -20,7 +20,6 @@
 // and would otherwise push the operand blocks, which every output block re-reads, out of L2.
 #include <algorithm>
 #include <memory>
-#include <numeric>
 
 #include "cq_internal.hpp"
 
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(128, 5) k_mult_nd4_warp(MultArgs M, const int*
 // (one per lane) and walks that row: its B block is staged once per step and read by all lanes as a broadcast.
 // That halves the bytes from L2 per pair and the shared-memory reads of B.  Two stages: these products have few
 // output blocks, so an SM holds few warps.  Measured (512-atom cell, into the H range, 24064 output blocks): 0.325 ms
-// against 0.473 for the warp-staged and 0.546 for the four-lanes-per-block kernel; into the L range (63664) 0.600
+// against 0.473 for the warp-staged and 0.378 for the four-lanes-per-block kernel; into the L range (63664) 0.600
 // against 0.601; three and four stages 0.766 and 0.878 there (the pair lists lose the L1).
 // tile: (kh's row start in B, its end, first entry of trans_dest for the outputs, their number).
 template <bool EXACT, int STAGES>
@@ -476,15 +475,13 @@ __global__ void __launch_bounds__(64) k_mult_nd4_row(MultArgs M, const int4* __r
 }
 
 // Uniform 4 x 4 blocks, one thread per output block, operand blocks staged by the bulk-copy (TMA)
-// engine.  The warp-staged kernel spends per triple about two L1 wavefronts on its coalesced global
-// loads, two on the shared-memory stores and two on each lane's shared-memory reads; here every lane
-// issues two 128-byte cp.async.bulk copies (its X and B blocks) into its slot of the warp's stage,
+// engine: every lane issues two 128-byte cp.async.bulk copies (its X and B blocks) into its slot of the warp's stage,
 // whose mbarrier counts the bytes, so only the reads of the staged blocks go through the load/store
 // pipe.  Three stages per warp keep the copies of the next two steps in flight.  Every wait is bounded
 // (about a second; the error word is set and the warp stops).  The arithmetic is the warp-staged
-// kernel's, in the same order: the same bits.  Measured on the nine products of the 512-atom SZ LNV
-// call it runs at 1.48 TFLOP/s against 3.65 for the warp-staged kernel: 68 M copies of 128 B in
-// 2.59 ms on LS.L -> LSL is one copy per about 11 SM cycles, so the copy engine, not L1, bounds it.
+// kernel's, in the same order: the same bits.  The copy engine bounds it: 68 M copies of 128 B in 2.59 ms on
+// LS.L -> LSL of the 512-atom SZ cell, one per about 11 SM cycles (the warp-staged kernel takes 0.57 ms).  No rule
+// chooses it.
 constexpr int kBulkStages = 3;
 constexpr int kBulkSlot = 144;            // bytes per staged block (128 + 16: conflict-free 16-byte reads)
 
@@ -725,6 +722,7 @@ struct GroupShape {
   static constexpr int kStrideB = 32 * ((MAXND * MAXND * 8 + 8 + 31) / 32 | 1);
   static constexpr int kStage = kBlocks * (kStrideX + kStrideB);      // the X blocks, then the B blocks
   static constexpr int kWarpBytes = STAGES * kStage;
+  static_assert(2 * kWarpBytes <= 48 * 1024, "two warps fit the shared memory that every launch may take");
 };
 
 // n doubles at src (8-byte aligned) to the 16-byte aligned slot dst, by the LPB lanes l of a group; the data
@@ -1294,8 +1292,8 @@ static void allow_smem(System& S, K* kern, int bytes) {
   CQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
-// One launch of the FP64 product with kernel `variant` (0..3 and 5 for uniform 4 x 4 blocks with
-// 16-byte aligned operands; anything else runs the generic kernel).  All variants give the same
+// One launch of the FP64 product with kernel `variant` (0..6 for uniform 4 x 4 blocks with 16-byte aligned operands; for
+// anything else 4 is the group kernel and every other number the generic one).  All variants give the same
 // bits: they differ only in how the work is mapped onto the GPU.
 static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int variant, int exact, bool nd4) {
   cudaStream_t st = S.stream;
@@ -1388,7 +1386,6 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   } else if (variant == 4) {
     order = output_order(S, P);
     auto launch = [&](auto kern, int blocks, int warp_bytes) {
-      allow_smem(S, kern, 2 * warp_bytes);
       kern<<<(M.n_out + 2 * blocks - 1) / (2 * blocks), 64, 2 * warp_bytes, st>>>(M, order);
     };
     auto by_size = [&](auto type, auto ex) {
@@ -1400,7 +1397,8 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
         else if (S.max_nsf <= 13) launch(k_mult_group<TY, EX, 0, 13, LPB, ST>, 32 / LPB, GroupShape<13, LPB, ST>::kWarpBytes);
         else launch(k_mult_group<TY, EX, 0, 16, LPB, ST>, 32 / LPB, GroupShape<16, LPB, ST>::kWarpBytes);
       };
-      // four blocks per warp once they give every SM its 18 resident warps (see k_mult_group)
+      // four blocks per warp once they give every SM its 18 resident warps: past the 8,000 output blocks where the two
+      // shapes are equal (see k_mult_group)
       if (M.n_out >= 148 * 18 * 4) by_group(std::integral_constant<int, 8>{}, std::integral_constant<int, 1>{});
       else by_group(std::integral_constant<int, 16>{}, std::integral_constant<int, 2>{});
     };
@@ -1505,8 +1503,10 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
   if (S.prof.on) { ev0 = S.prof.get(); CQ_CUDA(cudaEventRecord(ev0, st)); }
   // fused multiply-add products of blocks larger than 8 x 8 run on the FP64 tensor cores: an m8n8k4 MMA
   // chains its four products into the accumulator as fused multiply-adds in k order, so the bits are
-  // those of the CUDA-core kernels (checked on B200), about three times faster on 13 x 13 blocks
-  // (unless a CUDA-core variant is forced with CQ_OPT_MULT_VARIANT)
+  // those of the CUDA-core kernels (checked on B200; unless a CUDA-core variant is forced with CQ_OPT_MULT_VARIANT).
+  // Tensor cores / group kernel with fused multiply-add, us: LS.L -> LSL of 64 DZP atoms 1396 / 1639, LS.S -> SLS of 216
+  // 1223 / 1409, 216 atoms 8, 12 -> 20 bohr 84 / 86, 16 x 16 blocks 176 / 236, 5 and 13 rows 267 / 324, 9 x 9 267 / 270,
+  // 4 and 13 rows 235 / 214 (type 1) and 180 / 202 (type 2), 656 output blocks of a cluster 12.5 / 26.7
   if (exact == kPrecFp64Tensor || (exact == 0 && S.max_nsf > 8 && S.mult_variant == kVariantAuto)) {
     if (dmma_short(S, P, M.n_out)) {
       const int grid = (M.n_out + 3) / 4;
