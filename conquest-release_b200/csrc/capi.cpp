@@ -247,10 +247,11 @@ int cq_mat_mult_batch(int n, cq_system* const* systems, const int* mult_type, co
                "batched products are FP64 (CQ_PREC_FP64 or CQ_PREC_FP64_FMA)");
       CQ_CHECK(a_dev[k] && b_dev[k] && c_dev[k], CQ_ERR_ARG, "null operand");
       ProductPlan& P = get_plan(sys->S, mult_type[k], ra[k], rb[k], rc[k]);
-      ensure_product_order(sys->S, P);   // on the system's own stream, before its event below
       items.push_back({&sys->S, &P, a_dev[k], b_dev[k], c_dev[k], precision[k] == CQ_PREC_FP64 ? 1 : 0});
       if (std::find(streams.begin(), streams.end(), sys->S.stream) == streams.end()) streams.push_back(sys->S.stream);
     }
+    if (!batch_of_small_blocks(items))     // the output orders, on each system's own stream, before its event below
+      for (const BatchItem& it : items) ensure_product_order(*it.S, *it.P);
     // one launch on the first system's stream, after the work already on every system's stream;
     // every system's later work waits for it
     cudaStream_t st = streams[0];

@@ -64,9 +64,8 @@ __device__ __forceinline__ int ordered(const int* __restrict__ order, int slot) 
 // Measured (6298 output blocks, type 2, 47 terms each; us): 5 x 5 blocks 50.3, without the look-ahead 99.5 and 113.2
 // for the group kernel; blocks of 1 and 4 rows 55.6, 76.0 and 86.2.
 template <int TYPE, bool EXACT, int R>
-__global__ void __launch_bounds__(256) k_mult_generic(MultArgs M, int u) {
-  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (q >= M.n_out) return;
+__device__ __forceinline__ void warp_generic(const MultArgs& M, int u, int q) {
+  const int lane = threadIdx.x & 31;
   const int2* pairs = M.pairs + M.ptr[q];
   const int nt = (int)(M.ptr[q + 1] - M.ptr[q]);
   const int ndi = u ? u : M.prim_nsf[M.o_row[q]];
@@ -123,6 +122,12 @@ __global__ void __launch_bounds__(256) k_mult_generic(MultArgs M, int u) {
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (lane + 32 * r < ne) O[lane + 32 * r] = acc[r];
+}
+
+template <int TYPE, bool EXACT, int R>
+__global__ void __launch_bounds__(256) k_mult_generic(MultArgs M, int u) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q < M.n_out) warp_generic<TYPE, EXACT, R>(M, u, q);
 }
 
 // 4 x 4 blocks (SZ basis): 16 lanes per output block, one element per lane.  Each lane
@@ -1101,8 +1106,8 @@ __global__ void __launch_bounds__(128) k_mult_dmma_short(MultArgs M) {
 
 // Many independent products in one persistent launch (the concatenation of their output-block
 // lists): every warp takes work units u = warp id, warp id + warps in the grid, ...; a unit is 32
-// output slots of a uniform 4 x 4 product (the warp-staged kernel) or two output blocks of any other
-// product (the group kernel with 16 lanes per block).  Each output block is computed by exactly the operations
+// output slots of a uniform 4 x 4 product (the warp-staged kernel) or two output blocks of any other product (the group
+// kernel with 16 lanes per block), or one output block where all products are of small blocks (the generic kernel).  Each output block is computed by exactly the operations
 // of the single-product kernels, so the results are the same bits as separate launches.  The product table
 // travels in the kernel's parameters (no host-to-device copy before the launch).  Eight systems of 64 to 300 atoms
 // (1.98 GFLOP): 0.284 ms, against 0.684 ms with one output block per warp and register tiles of 4 x 2.
@@ -1110,6 +1115,7 @@ struct BatchProduct {
   MultArgs M;
   const int* order;                // output blocks by descending pair count
   int kind;                        // bit 0: type 2, bit 1: exact rounding, bits 2..: kBatchNd4, ...
+  int u;                           // the block size when the whole system has one, else 0
 };
 enum { kBatchNd4 = 0, kBatchU13 = 4, kBatchMax13 = 8, kBatchMax16 = 12 };
 constexpr int kBatchMax = 96;      // products per launch (the table stays within the 32 KB parameter space)
@@ -1124,9 +1130,11 @@ constexpr int kBatchWarpBytes = kStageBytes + 256;    // the larger of the two k
 static_assert(GroupShape<13, 16, 1>::kWarpBytes <= kBatchWarpBytes && GroupShape<16, 16, 1>::kWarpBytes <= kBatchWarpBytes,
               "batched warps share one staging area");
 
-template <int TYPE, bool EXACT>
+template <int TYPE, bool EXACT, bool SMALL>
 __device__ __forceinline__ void batch_unit(const BatchProduct& P, int family, int unit, unsigned char* W) {
-  if (family == kBatchNd4) {
+  if constexpr (SMALL) {
+    warp_generic<TYPE, EXACT, 1>(P.M, P.u, unit);
+  } else if (family == kBatchNd4) {
     warp_nd4_staged<TYPE, EXACT>(P.M, P.order, unit * 32, W);
   } else if (family == kBatchU13) {
     warp_group<TYPE, EXACT, 13, 13, 16, 1>(P.M, P.order, unit * 2, W);
@@ -1137,8 +1145,10 @@ __device__ __forceinline__ void batch_unit(const BatchProduct& P, int family, in
   }
 }
 
+// SMALL: every product is of small blocks (batch_of_small_blocks)
+template <bool SMALL>
 __global__ void __launch_bounds__(128, 4) k_mult_batch(const __grid_constant__ BatchParams B) {
-  __shared__ __align__(128) unsigned char smem[4][kBatchWarpBytes];
+  __shared__ __align__(128) unsigned char smem[4][SMALL ? 16 : kBatchWarpBytes];
   const int warp = threadIdx.x >> 5;
   const int n_units = B.unit_off[B.n_prod];
   for (int u = blockIdx.x * 4 + warp; u < n_units; u += gridDim.x * 4) {
@@ -1150,10 +1160,10 @@ __global__ void __launch_bounds__(128, 4) k_mult_batch(const __grid_constant__ B
     const BatchProduct& P = B.prods[lo];
     const int family = P.kind & ~3, unit = u - B.unit_off[lo];
     switch (P.kind & 3) {
-      case 0: batch_unit<1, false>(P, family, unit, smem[warp]); break;
-      case 1: batch_unit<2, false>(P, family, unit, smem[warp]); break;
-      case 2: batch_unit<1, true>(P, family, unit, smem[warp]); break;
-      default: batch_unit<2, true>(P, family, unit, smem[warp]); break;
+      case 0: batch_unit<1, false, SMALL>(P, family, unit, smem[warp]); break;
+      case 1: batch_unit<2, false, SMALL>(P, family, unit, smem[warp]); break;
+      case 2: batch_unit<1, true, SMALL>(P, family, unit, smem[warp]); break;
+      default: batch_unit<2, true, SMALL>(P, family, unit, smem[warp]); break;
     }
     __syncwarp();                                // the staging area goes to the next unit
   }
@@ -1544,6 +1554,17 @@ void launch_mat_mult(System& S, ProductPlan& P, double* a, const double* b, doub
 
 void ensure_product_order(System& S, ProductPlan& P) { output_order(S, P); }
 
+// A batch whose products are all of small blocks (other than aligned 4 x 4) runs the generic kernel, in the stored order.
+// Six products of a system, us, group / generic: 60 atoms of 1 and 4 rows (3548 and 1014 output blocks) 82.8 / 54.8, of 5 x 5
+// 107.9 / 55.3, 150 atoms of 1 x 1 (4432, 624) 17.5 / 10.9; but 16,676 and 3016 of 1 x 1 119.7 / 132.2.  One kernel per call:
+// next to the other bodies the generic one made the registers of all spill (every other product a third slower), and two
+// launches in a row lose what their overlap gives.
+bool batch_of_small_blocks(const std::vector<BatchItem>& items) {
+  for (const BatchItem& it : items)
+    if (it.S->uniform_nsf == 4 || it.S->max_nsf > 5 || it.S->ranges[it.P->out_range]->nnz >= 10000) return false;
+  return true;
+}
+
 // Products of independent systems (or of one system) in persistent launches on `st` (up to kBatchMax
 // products each).  The caller orders `st` after the work the operands depend on and the systems' later
 // work after it.
@@ -1551,14 +1572,16 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
   int dev_id = 0, sms = 0, occ = 0;
   CQ_CUDA(cudaGetDevice(&dev_id));
   CQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id));
-  CQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mult_batch, 128, 0));
+  const bool small = batch_of_small_blocks(items);
   auto params = std::make_unique<BatchParams>();
   BatchParams& B = *params;
   auto flush = [&] {
     if (B.n_prod == 0) return;
     const int n_units = B.unit_off[B.n_prod];
+    auto* kern = small ? k_mult_batch<true> : k_mult_batch<false>;
+    CQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 128, 0));
     const int grid = std::max(1, std::min(sms * std::max(occ, 1), (n_units + 3) / 4));
-    k_mult_batch<<<grid, 128, 0, st>>>(B);
+    kern<<<grid, 128, 0, st>>>(B);
     CQ_CUDA(cudaGetLastError());
     B.n_prod = 0;
   };
@@ -1574,9 +1597,11 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
     bp.order = P.order.p;              // built by ensure_product_order on the system's stream; null under capture
     bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) |
               (nd4 ? kBatchNd4 : S.uniform_nsf == 13 ? kBatchU13 : S.max_nsf <= 13 ? kBatchMax13 : kBatchMax16);
+    bp.u = S.uniform_nsf;
     if (B.n_prod == kBatchMax) { flush(); B.unit_off[0] = 0; }
     B.prods[B.n_prod] = bp;
-    B.unit_off[B.n_prod + 1] = B.unit_off[B.n_prod] + (nd4 ? (bp.M.n_out + 31) / 32 : (bp.M.n_out + 1) / 2);
+    const int per_unit = small ? 1 : nd4 ? 32 : 2;
+    B.unit_off[B.n_prod + 1] = B.unit_off[B.n_prod] + (bp.M.n_out + per_unit - 1) / per_unit;
     ++B.n_prod;
     S.launches++;
   }

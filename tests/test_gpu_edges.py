@@ -201,3 +201,36 @@ def test_row_kernel_builds_no_output_order():
     g.mat_mult(2, 0, 1, 2, *ops)
     g.synchronize()
     assert g.launch_count() - before == 1
+
+
+@pytest.mark.parametrize("tables", [("u4",), ("1_4",), ("u4", "1_4", "u13", "5_13", "u16", "u2"), ("u2", "u4")])
+@pytest.mark.parametrize("exact", [True, False])
+def test_batches_of_small_and_other_blocks(tables, exact):
+    """Batches of 4 x 4 products alone (their own kernel), of small blocks alone and of every kind in one table, both mult
+    types, few and many output blocks: the bits of the separate products."""
+    import torch
+    import cq_b200
+    items, outs, keep = [], [], []
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(23)
+    for k, name in enumerate(tables):
+        sizes = [int(x) for x in name.lstrip("u").split("_")]
+        for coords, cell in (inputs.si_cluster(21 + k, sigma=0.1, seed=97), inputs.diamond_si(2, sigma=0.05, seed=98)):
+            nsf = np.array([sizes[i % len(sizes)] for i in range(len(coords))], np.int32)
+            g = cq_b200.System(coords, cell, nsf, [7.0, 6.0, 13.0])
+            keep.append(g)
+            for t in (1, 2):
+                ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for r in range(3)]
+                o = 2 if t == 1 else 0
+                torch.cuda.synchronize()
+                g.mat_mult(t, 0, 1, 2, *ops, exact=exact)
+                g.synchronize()
+                outs.append((ops[o], ops[o].clone()))
+                ops[o].fill_(float("nan"))
+                items.append((g, t, 0, 1, 2, *ops, int(exact)))
+    torch.cuda.synchronize()
+    cq_b200.mat_mult_batch(items)
+    for g in keep:
+        g.synchronize()
+    for got, want in outs:
+        assert torch.equal(got, want)
