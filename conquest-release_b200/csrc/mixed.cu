@@ -323,14 +323,14 @@ static void mat_mult_mma_sync(System& S, MixedPlan& MP, int mult_type, int ra, i
 // so that a product always runs the same kernel (and gives the same bits) whatever else runs on the device.  Two costs
 // are compared:
 //  - a block per mma.sync warp: 18 us and a time per pair, which is that of the 2 KB of fragments it fetches: 105 to
-//    118 ps with B's fragments (1 KB per block) well inside the L2, 125 to 151 ps where they are as large as it
-//    (112 and 143 below);
+//    118 ps with B's fragments (1 KB per block) well inside the L2, 125 to 151 ps where they are as large as it, 148 ps at
+//    four times its size (112, 143 and 148 below);
 //  - tcgen05 tiles: 40 us and the tensor work they issue, at 690 to 890 TFLOP/s once there are a few hundred tiles
 //    (820 below).
 // The tiles are taken only where at least kTileMinFill of that work is useful: the bound that this choice has always had
 // (dense products of 4 x 4 blocks lie under it and would gain: 2288 / 208 us on a 300-atom cluster at 32 bohr).
 // Measured in us, blocks / tiles: LS.L -> LSL of DZP cells (26, 16 -> 42 bohr) 216 atoms 1549 / 2162, 512 atoms 4004 /
-// 4897, 1000 atoms 9267 / 8615, 1728 atoms 16655 / 14643; 20, 20 -> 40 bohr 512 atoms 5439 / 5040, 1000 atoms 10891 / 8941;
+// 4897, 1000 atoms 9267 / 8615, 1728 atoms 16655 / 14643, 4096 atoms 40,200 / 39,500; 20, 20 -> 40 bohr 512 atoms 5439 / 5040, 1000 atoms 10891 / 8941;
 // 300-atom clusters (16, 16) 236 / 270, (20, 20) 594 / 499, (32, 32) 2387 / 1252, and of 4- and 13-orbital atoms
 // 2318 / 470; 100 atoms (16, 16) 55 / 66, (20, 20) 91 / 79.
 constexpr double kTileMinFill = 0.11;
@@ -339,7 +339,8 @@ constexpr int64_t kTileMinPairs = 300000;     // fewer never pay: no estimate of
 bool split_tiles_pay(int64_t n_pairs, int64_t flops, double issued_flops, int64_t b_blocks) {
   if (n_pairs < kTileMinPairs || issued_flops <= 0.0 || 3.0 * (double)flops < kTileMinFill * issued_flops) return false;
   const double mb = (double)b_blocks * 1024e-6;
-  const double ps = 112.0 + 31.0 * std::min(std::max((mb - 64.0) / (127.0 - 64.0), 0.0), 1.0);
+  auto part = [&](double from, double to) { return std::min(std::max((mb - from) / (to - from), 0.0), 1.0); };
+  const double ps = 112.0 + 31.0 * part(64.0, 127.0) + 5.0 * part(127.0, 500.0);
   return 40e-6 + issued_flops / 820e12 < 18e-6 + (double)n_pairs * ps * 1e-12;
 }
 

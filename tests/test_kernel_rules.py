@@ -13,6 +13,8 @@ MEASURED = {
     "c1000_dzp_26_16": (66.27e6, 291.3e9, 6827e9, 124350, TILES),       # 9267 / 8615
     "c1000_dzp_26_16_t2": (66.28e6, 291.3e9, 8244e9, 124350, BLOCKS),   # 8683 / 10494
     "c1728_dzp_26_16": (114.5e6, 503.7e9, 11714e9, 214900, TILES),      # 16655 / 14643
+    "c4096_dzp_26_16": (271.5e6, 1193e9, 31580e9, 509000, TILES),       # 40200 / 39500
+    "k1500_dzp_22_16_t2": (33.3e6, 146.4e9, 3960e9, 141400, BLOCKS),    # 3931 / 4581
     "c216_dzp_26_16": (14.31e6, 62.9e9, 1497e9, 26830, BLOCKS),         # 1549 / 2162
     "k300_dzp_16": (1.786e6, 7.85e9, 181e9, 22140, BLOCKS),             # 236 / 270
     "k300_dzp_20": (5.681e6, 24.97e9, 446e9, 39766, TILES),             # 594 / 499
