@@ -546,9 +546,8 @@ struct CoverTiling {
   std::vector<int> nd_prim;                         // block size of each primary atom
   std::vector<int> unit_of, unit_pos;               // cover atom -> unit, position in it
   std::vector<int> chunk_of, chunk_pos, chunk_first;
-  std::vector<unsigned int> ktab;                   // [unit][16]
   std::vector<int> grp_first;                       // at most kM rows and kMaxAtoms atoms each
-  int n_units() const { return (int)(ktab.size() / kUK); }
+  int n_units = 0;
   int n_chunks() const { return (int)chunk_first.size() - 1; }
   int n_groups() const { return (int)grp_first.size() - 1; }
 };
@@ -562,11 +561,11 @@ CoverTiling cover_tiling(const Geometry& g) {
   int u = -1, uw = kUK + 1, ua = kMaxUnitAtoms;
   for (int c = 0; c < ncov; ++c) {
     const int nd = g.cover_nsf[c];
-    if (uw + nd > kUK || ua == kMaxUnitAtoms) { ++u; uw = 0; ua = 0; t.ktab.resize((size_t)(u + 1) * kUK, 0xffffffffu); }
-    for (int o = 0; o < nd; ++o) t.ktab[(size_t)u * kUK + uw + o] = (unsigned)ua | ((unsigned)o << 8) | ((unsigned)nd << 16);
+    if (uw + nd > kUK || ua == kMaxUnitAtoms) { ++u; uw = 0; ua = 0; }
     t.unit_of[c] = u; t.unit_pos[c] = ua;
     uw += nd; ++ua;
   }
+  t.n_units = u + 1;
   for (int c = 0, w = kNT + 1, cnt = kMaxAtoms; c < ncov; ++c) {
     const int nd = g.cover_nsf[c];
     if (w + nd > kNT || cnt == kMaxAtoms) { t.chunk_first.push_back(c); w = 0; cnt = 0; }
@@ -595,6 +594,8 @@ __global__ void k_umma_sample(int q0, int q1, const int64_t* __restrict__ ptr, c
   for (int64_t p = ptr[q] + lane; p < ptr[q + 1]; p += 32) {
     const int64_t bit = base + unit_of[xcov[pairs[p].x]];
     const unsigned m = 1u << (bit & 31);
+    // bits are only ever set: one that is seen needs no atomic (about fourteen pairs share a bit)
+    if (*(volatile unsigned int*)(bits + (bit >> 5)) & m) continue;
     if (!(atomicOr(bits + (bit >> 5), m) & m)) ++n;
   }
   n = __reduce_add_sync(0xffffffffu, n);
@@ -615,7 +616,7 @@ double umma_issued_estimate(System& S, int mult_type, int ra, int rb, int rc) {
   if (O.nnz == 0 || !umma_usable(S)) return 0.0;
   const CoverTiling ct = cover_tiling(S.geo);
   const int ng = ct.n_groups(), ns = std::min(ng, 12);
-  const int64_t words = ((int64_t)ct.n_units() * ct.n_chunks() + 31) / 32;
+  const int64_t words = ((int64_t)ct.n_units * ct.n_chunks() + 31) / 32;
   if (words > (int64_t)1 << 28) return 0.0;         // 1 GiB of marks
   cudaStream_t st = S.stream;
   DevBuf<int> unit_of, chunk_of;
@@ -632,7 +633,7 @@ double umma_issued_estimate(System& S, int mult_type, int ra, int rb, int rc) {
     if (q0 == q1) continue;
     CQ_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned int) * words, st));
     k_umma_sample<<<(int)(((int64_t)(q1 - q0) * 32 + 255) / 256), 256, 0, st>>>(
-        q0, q1, P.ptr.p, P.pairs.p, X.nb_cover.p, O.nb_cover.p, unit_of.p, chunk_of.p, ct.n_units(), bits.p, counts.p);
+        q0, q1, P.ptr.p, P.pairs.p, X.nb_cover.p, O.nb_cover.p, unit_of.p, chunk_of.p, ct.n_units, bits.p, counts.p);
     CQ_CUDA(cudaGetLastError());
     S.launches++;
   }
@@ -663,8 +664,15 @@ UmmaPlan& get_umma_plan(System& S, int mult_type, int ra, int rb, int rc) {
   CoverTiling ct = cover_tiling(g);
   const std::vector<int>&nd_prim = ct.nd_prim, &chunk_first = ct.chunk_first, &grp_first = ct.grp_first;
   std::vector<int>&unit_of = ct.unit_of, &unit_pos = ct.unit_pos, &chunk_of = ct.chunk_of, &chunk_pos = ct.chunk_pos;
-  std::vector<unsigned int>& ktab = ct.ktab;
-  const int n_units = ct.n_units(), n_chunks = ct.n_chunks(), ng = ct.n_groups();
+  const int n_units = ct.n_units, n_chunks = ct.n_chunks(), ng = ct.n_groups();
+  std::vector<unsigned int> ktab((size_t)n_units * kUK, 0xffffffffu);   // [unit][16]: the orbitals of its atoms
+  for (int c = 0, w = 0; c < g.n_cover_atoms; ++c) {
+    const int nd = g.cover_nsf[c];
+    if (unit_pos[c] == 0) w = 0;
+    for (int o = 0; o < nd; ++o)
+      ktab[(size_t)unit_of[c] * kUK + w + o] = (unsigned)unit_pos[c] | ((unsigned)o << 8) | ((unsigned)nd << 16);
+    w += nd;
+  }
   // host copies of the output and first-operand neighbour lists
   std::vector<int> ocov(O.nnz), xcov(std::max(X.nnz, 1));
   CQ_CUDA(cudaMemcpyAsync(ocov.data(), O.nb_cover.p, sizeof(int) * O.nnz, cudaMemcpyDeviceToHost, st));
