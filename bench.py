@@ -556,8 +556,9 @@ def main():
             "parity": fixture_parity(res),
             "mixed_vs_fp64": mixed,
             "block_mult_tflops": (prof["flops"] / (prof["ms"] / 1e3) / 1e12) if prof["ms"] > 0 else None,
-            "roofline": {"bound": "hbm", "kernel": "FP64 4x4 block products (k_mult_nd4_warp / _row / _quad, chosen by size)", "achieved": achieved,
-                         "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
+            "roofline": {"bound": "l2", "kernel": "FP64 4x4 block products (k_mult_nd4_warp / _row / _quad, chosen by size)", "achieved": achieved,
+                         "peak": peak, "peak_kind": peak_kind + "; the products are bound by operand blocks from L2, not by HBM",
+                         "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic[0], "traffic_launch": traffic[1],
                          "traffic_launch_algorithmic_bytes": traffic[2], "launches": prof["launches"],
                          "avg_launch_ms": prof["ms"] / max(1, prof["launches"]),

@@ -61,7 +61,8 @@ def main():
     g.mat_mult(1, 0, 1, 2, da, db, dc)
     g.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    st = torch.cuda.current_stream()
+    st = torch.cuda.Stream()              # a stream of its own: the default one's handle, 0, would mean the system's
+    torch.cuda.synchronize()
     g.set_stream(st.cuda_stream)
     e0.record(st)
     for _ in range(5):
