@@ -353,6 +353,7 @@ struct BatchItem {                 // one FP64 product of a batched launch (role
 };
 void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st);
 bool batch_of_small_blocks(const std::vector<BatchItem>& items);   // runs without output orders
+bool capturing(const System& S);  // the system's stream is being captured into a graph: nothing may wait or allocate
 void ensure_product_order(System& S, ProductPlan& P);   // the staged kernels' output order (built once)
 
 // gen.cu: synthetic S (which = 0) or H (which = 1) of range r into out

@@ -350,6 +350,7 @@ void mat_mult_mixed(System& S, int mult_type, int ra, int rb, int rc, double* a,
   int k = S.mixed_kernel;
   if (parts == 3) k = 1;
   if (k == 0 && !umma_usable(S)) k = 1;
+  if (k < 0 && MP.kernel < 0 && capturing(S)) k = 1;   // the estimate below waits for the stream: no choice is recorded
   if (k < 0) {
     if (MP.kernel < 0) {
       MP.kernel = 1;

@@ -1260,7 +1260,7 @@ __global__ void __launch_bounds__(256) k_order_fill(OrderKey key, int n, int bin
 }
 }  // namespace
 
-static bool capturing(const System& S) {
+bool capturing(const System& S) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   CQ_CUDA(cudaStreamIsCapturing(S.stream, &status));
   return status != cudaStreamCaptureStatusNone;

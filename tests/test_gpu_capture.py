@@ -60,3 +60,33 @@ def test_first_call_inside_a_capture(sizes, precision, variant, batch, mult_type
         g.close()
     assert not torch.isnan(outs[0]).any()
     assert torch.equal(outs[0], outs[1])
+
+
+def test_two_part_split_captured_before_its_kernel_is_chosen():
+    """A two-part split product whose fragments and lists exist (from a three-part call) but whose kernel has not been chosen:
+    the captured call runs on the blocks, a later direct one chooses (tiles, on this dense cluster)."""
+    import torch
+    import cq_b200
+    coords, cell = inputs.si_cluster(100, sigma=0.1, seed=2, vacuum=15.0)
+    g = cq_b200.System(coords, cell, np.full(len(coords), 13, np.int32), [20.0, 20.0, 40.0])
+    stream = torch.cuda.Stream()
+    g.set_stream(stream.cuda_stream)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(19)
+    ops = [torch.rand(g.length(r), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for r in range(3)]
+    torch.cuda.synchronize()
+    g.mat_mult(1, 0, 1, 2, *ops, precision=cq_b200.PREC_BF16X6)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        g.mat_mult(1, 0, 1, 2, *ops, precision=cq_b200.PREC_BF16X3)
+    ops[2].fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    captured = ops[2].clone()
+    outs = {}
+    for k in (-1, 0, 1):
+        g.set_mixed_kernel(k)
+        g.mat_mult(1, 0, 1, 2, *ops, precision=cq_b200.PREC_BF16X3)
+        g.synchronize()
+        outs[k] = ops[2].clone()
+    assert torch.equal(captured, outs[1]) and torch.equal(outs[-1], outs[0]) and not torch.equal(outs[0], outs[1])
