@@ -53,7 +53,8 @@ struct MultArgs {
   double* __restrict__ out;
 };
 
-// Output block at a slot of the launch: the plan's order where it has been built, else the stored order.
+// Output block at a slot of the launch: the plan's order where it has been built, else the stored order.  (The 4 x 4 kernels
+// always have the order: the test alone costs their smallest products 3 %.)
 __device__ __forceinline__ int ordered(const int* __restrict__ order, int slot) { return order ? order[slot] : slot; }
 
 // Any block sizes (nd <= 16): one warp per output block, R elements per lane (32 R >= the largest block), operands read
@@ -341,7 +342,7 @@ __device__ __forceinline__ void warp_nd4_staged(const MultArgs& M, const int* __
   const int lane = threadIdx.x & 31;
   const int slot = base + lane;
   const bool has = slot < M.n_out;
-  const int q = has ? ordered(order, slot) : 0;
+  const int q = has ? order[slot] : 0;
   const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
   const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
   const int steps = __reduce_max_sync(kFull, nt);
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(128, 2) k_mult_nd4_bulk(MultArgs M, const int*
   if (base >= M.n_out) return;                  // whole warp (nothing waits on its barriers)
   const int slot = base + lane;
   const bool has = slot < M.n_out;
-  const int q = has ? ordered(order, slot) : 0;
+  const int q = has ? order[slot] : 0;
   const int64_t t = has ? M.ptr[q] : 0;
   const int64_t tend = has ? M.ptr[q + 1] : 0;
   double acc[16];
@@ -630,7 +631,7 @@ __global__ void __launch_bounds__(128) k_mult_nd4_quad(MultArgs M, const int* __
   if (base >= M.n_out) return;                   // whole warp
   const int slot = base + qd;
   const bool has = slot < M.n_out;
-  const int q = has ? ordered(order, slot) : 0;
+  const int q = has ? order[slot] : 0;
   const int2* pairs = M.pairs + (has ? M.ptr[q] : 0);
   const int nt = has ? (int)(M.ptr[q + 1] - M.ptr[q]) : 0;
   const int steps = __reduce_max_sync(kFull, nt);
@@ -1310,10 +1311,11 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   const int T = 256;
   RangeIndex& O = P.mult_type == 1 ? *S.ranges[P.rc] : *S.ranges[P.ra];
   RangeIndex& X = P.mult_type == 1 ? *S.ranges[P.ra] : *S.ranges[P.rc];
-  // the row kernel's tiles are uploaded on its first use: a launch captured before then takes the warp-staged kernel
+  // the row kernel's tiles are uploaded on its first use: a launch captured before then takes another kernel
   if (nd4 && variant == 4 && P.mult_type == 2 && P.n_row_tiles < 0 && capturing(S)) variant = 3;
   const bool row_kernel = nd4 && variant == 4 && P.mult_type == 2;        // the row kernel has an order of its own
   const int* order = nd4 && variant >= 3 && !row_kernel ? output_order(S, P) : nullptr;
+  if (nd4 && variant >= 3 && !row_kernel && !order) variant = 0;       // captured before the order exists
   if (nd4 && variant == 6) {
     const int grid = (M.n_out + 127) / 128;
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
@@ -1595,6 +1597,7 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
     bp.M = product_args(S, P, it.a, it.b, it.c, &nd4);
     if (bp.M.n_out == 0) continue;
     bp.order = P.order.p;              // built by ensure_product_order on the system's stream; null under capture
+    nd4 = nd4 && bp.order;             // the 4 x 4 body needs it, the group body does not
     bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) |
               (nd4 ? kBatchNd4 : S.uniform_nsf == 13 ? kBatchU13 : S.max_nsf <= 13 ? kBatchMax13 : kBatchMax16);
     bp.u = S.uniform_nsf;

@@ -14,7 +14,8 @@ SIZES = {"u13": lambda k: 13, "4_13": lambda k: 13 if k % 3 == 0 else 4, "u4": l
 @pytest.mark.parametrize("mult_type", [1, 2])
 @pytest.mark.parametrize("sizes,precision,variant,batch", [
     ("u13", "PREC_FP64_TC", -1, False), ("4_13", "PREC_FP64_FMA", -1, False), ("u13", "PREC_FP64", 4, False),
-    ("4_13", "PREC_FP64", 4, True), ("u4", "PREC_FP64", 4, False), ("u4", "PREC_FP64", 5, False)])
+    ("4_13", "PREC_FP64", 4, True), ("u4", "PREC_FP64", 4, False), ("u4", "PREC_FP64", 5, False), ("u4", "PREC_FP64", -1, False),
+    ("u4", "PREC_FP64_FMA", 6, False), ("u4", "PREC_FP64", -1, True)])
 def test_first_call_inside_a_capture(sizes, precision, variant, batch, mult_type):
     import torch
     import cq_b200
