@@ -53,10 +53,6 @@ struct MultArgs {
   double* __restrict__ out;
 };
 
-// Output block at a slot of the launch: the plan's order where it has been built, else the stored order.  (The 4 x 4 kernels
-// always have the order: the test alone costs their smallest products 3 %.)
-__device__ __forceinline__ int ordered(const int* __restrict__ order, int slot) { return order ? order[slot] : slot; }
-
 // Any block sizes (nd <= 16): one warp per output block, R elements per lane (32 R >= the largest block), operands read
 // from global memory.  What bounds it: the chain of dependent loads of a pair (pair list, block offsets, inner dimension,
 // values), so the next pair's offsets are looked up while the current one's values are on their way, and the list is read
@@ -806,7 +802,7 @@ __device__ __forceinline__ void warp_group_rows(const MultArgs& M, const int* __
   const unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31, g = lane / LPB, l = lane % LPB;
   const bool has = base + g < M.n_out;
-  const int q = has ? ordered(order, base + g) : 0;
+  const int q = has ? order[base + g] : 0;
   const int ndi = FULL ? R : M.prim_nsf[M.o_row[q]];
   const int ndo = U > 0 ? U : M.cover_nsf[M.o_cover[q]];     // type 1: nd_j ; type 2: nd_k
   int c[H];
@@ -899,7 +895,7 @@ __device__ __forceinline__ void warp_group(const MultArgs& M, const int* __restr
     // several sizes: a warp whose blocks all have four rows, or all MAXND, runs a tile of exactly that height
     // (the order keeps blocks of one row count together)
     const int s = min(base + (threadIdx.x & 31) / LPB, M.n_out - 1);
-    const int ndi = M.prim_nsf[M.o_row[ordered(order, s)]];
+    const int ndi = M.prim_nsf[M.o_row[order[s]]];
     if (__all_sync(0xffffffffu, ndi == 4)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, 4, true>(M, order, base, W);
     else if (__all_sync(0xffffffffu, ndi == MAXND)) warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, true>(M, order, base, W);
     else warp_group_rows<TYPE, EXACT, 0, MAXND, LPB, STAGES, MAXND, false>(M, order, base, W);
@@ -945,7 +941,7 @@ __global__ void __launch_bounds__(64) k_mult_dmma(MultArgs M, const int* __restr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = blockIdx.x * 2 + warp;
   if (slot >= M.n_out) return;                    // whole warp
-  const int q = ordered(order, slot);
+  const int q = order ? order[slot] : slot;      // null: the stored order
   const int g = lane >> 2, t = lane & 3;          // fragment row / column and contraction index
   const int gp = lane >> 3, l = lane & 7;         // staging: pair and lane of its group
   unsigned char* W = smem[warp];
@@ -1267,8 +1263,8 @@ bool capturing(const System& S) {
   return status != cudaStreamCaptureStatusNone;
 }
 
-// The plan's output order, built on its first use, which allocates: a launch that is being
-// captured into a graph before then runs in the stored order instead (null: the same results).
+// The plan's output order, built on its first use, which allocates: null for a launch that is being captured into a graph
+// before then.
 static const int* output_order(System& S, ProductPlan& P) {
   const RangeIndex& O = *S.ranges[P.out_range];
   if (P.order.n != 0 || O.nnz == 0 || capturing(S)) return P.order.p;
@@ -1303,6 +1299,25 @@ static void allow_smem(System& S, K* kern, int bytes) {
   CQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
+// The generic kernel, which needs no output order: 32 R elements per block.
+static void launch_generic(const System& S, const ProductPlan& P, const MultArgs& M, int exact, cudaStream_t st) {
+  const int T = 256, grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
+  auto by_type = [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    if (P.mult_type == 1) {
+      if (exact) k_mult_generic<1, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+      else k_mult_generic<1, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+    } else {
+      if (exact) k_mult_generic<2, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+      else k_mult_generic<2, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
+    }
+  };
+  if (S.max_nsf <= 5) by_type(std::integral_constant<int, 1>{});
+  else if (S.max_nsf <= 8) by_type(std::integral_constant<int, 2>{});
+  else by_type(std::integral_constant<int, 8>{});
+  CQ_CUDA(cudaGetLastError());
+}
+
 // One launch of the FP64 product with kernel `variant` (0..6 for uniform 4 x 4 blocks with 16-byte aligned operands; for
 // anything else 4 is the group kernel and every other number the generic one).  All variants give the same
 // bits: they differ only in how the work is mapped onto the GPU.
@@ -1314,8 +1329,10 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
   // the row kernel's tiles are uploaded on its first use: a launch captured before then takes another kernel
   if (nd4 && variant == 4 && P.mult_type == 2 && P.n_row_tiles < 0 && capturing(S)) variant = 3;
   const bool row_kernel = nd4 && variant == 4 && P.mult_type == 2;        // the row kernel has an order of its own
-  const int* order = nd4 && variant >= 3 && !row_kernel ? output_order(S, P) : nullptr;
-  if (nd4 && variant >= 3 && !row_kernel && !order) variant = 0;       // captured before the order exists
+  // the staged kernels take their output order without a test for its absence (the test alone cost the smallest products
+  // 2 to 4 %): a launch captured before the order exists runs variant 0, which has none
+  const int* order = nullptr;
+  if ((nd4 ? variant >= 3 && !row_kernel : variant == 4) && !(order = output_order(S, P))) variant = 0;
   if (nd4 && variant == 6) {
     const int grid = (M.n_out + 127) / 128;
     const size_t smem = (size_t)4 * kBulkStages * 64 * kBulkSlot;
@@ -1396,7 +1413,6 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) k_mult_nd4<2, true><<<grid, T, 0, st>>>(M); else k_mult_nd4<2, false><<<grid, T, 0, st>>>(M);
     }
   } else if (variant == 4) {
-    order = output_order(S, P);
     auto launch = [&](auto kern, int blocks, int warp_bytes) {
       kern<<<(M.n_out + 2 * blocks - 1) / (2 * blocks), 64, 2 * warp_bytes, st>>>(M, order);
     };
@@ -1421,18 +1437,7 @@ static void launch_variant(System& S, ProductPlan& P, const MultArgs& M, int var
       if (exact) by_size(integral_constant<int, 2>{}, std::true_type{}); else by_size(integral_constant<int, 2>{}, std::false_type{});
     }
   } else {
-    const int grid = (int)(((int64_t)M.n_out * 32 + T - 1) / T);
-    auto by_type = [&](auto r) {
-      constexpr int R = decltype(r)::value;
-      if (P.mult_type == 1) {
-        if (exact) k_mult_generic<1, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf); else k_mult_generic<1, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
-      } else {
-        if (exact) k_mult_generic<2, true, R><<<grid, T, 0, st>>>(M, S.uniform_nsf); else k_mult_generic<2, false, R><<<grid, T, 0, st>>>(M, S.uniform_nsf);
-      }
-    };
-    if (S.max_nsf <= 5) by_type(std::integral_constant<int, 1>{});
-    else if (S.max_nsf <= 8) by_type(std::integral_constant<int, 2>{});
-    else by_type(std::integral_constant<int, 8>{});
+    launch_generic(S, P, M, exact, st);
   }
   S.launches++;
   CQ_CUDA(cudaGetLastError());
@@ -1596,8 +1601,12 @@ void launch_mat_mult_batch(const std::vector<BatchItem>& items, cudaStream_t st)
     BatchProduct bp;
     bp.M = product_args(S, P, it.a, it.b, it.c, &nd4);
     if (bp.M.n_out == 0) continue;
-    bp.order = P.order.p;              // built by ensure_product_order on the system's stream; null under capture
-    nd4 = nd4 && bp.order;             // the 4 x 4 body needs it, the group body does not
+    bp.order = P.order.p;              // built by ensure_product_order on the system's stream
+    if (!small && !bp.order) {         // captured before it exists: a launch of its own
+      launch_generic(S, P, bp.M, it.exact, st);
+      S.launches++;
+      continue;
+    }
     bp.kind = (P.mult_type == 2 ? 1 : 0) | (it.exact ? 2 : 0) |
               (nd4 ? kBatchNd4 : S.uniform_nsf == 13 ? kBatchU13 : S.max_nsf <= 13 ? kBatchMax13 : kBatchMax16);
     bp.u = S.uniform_nsf;
